@@ -10,6 +10,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "nfx_internal.h"
@@ -133,6 +134,8 @@ void free_mesh(nfx_sim* s) {
     s->d_stage = nullptr;
     s->have_mesh = false;
 }
+
+int host_threads() { return (int)std::max(1u, std::thread::hardware_concurrency()); }
 
 // Kernel view of the one-cell table (no tile or block maps: everything is cell 0).
 BatchDev table_view(const nfx_sim* s) {
@@ -313,20 +316,27 @@ int nfx_plan_check(int64_t np, int64_t nt, const double* points, const uint32_t*
                 uses[loc]++;
             }
         }
-        // incidence list: node q's run holds exactly its corners, as corner-major slots, in order
-        uint32_t prev_count = 0xffffffffu;
+        // incidence lists: node q's run holds exactly its corners, each once, as byte offsets of the
+        // corner-major slots, eight entries apart and inside the tile's stride; the quarters (eight
+        // consecutive nodes) have falling counts
+        uint32_t prev_min = 0xffffffffu, quarter_min = 0xffffffffu;
         for (int64_t q = 0; q < nn; q++) {
             const uint32_t w = P.tile_nodes[2 * (b * NM + q) + 1], first = w >> 16, count = w & 0xffffu;
-            if ((int)count != uses[q] || count > prev_count) return bad("incidence counts");
-            prev_count = count;
-            int last = -1;
-            for (uint32_t e = 0; e < count; e++) {
-                const uint32_t v = P.tile_inc[4 * b * T + first + e], k = v / T, j = v % T;
-                if ((int64_t)j >= ntt || P.lconn[4 * (b * T + j) + k] != q) return bad("incidence entry");
-                const int order = (int)(4 * j + k);
-                if (order <= last) return bad("incidence order");
-                last = order;
+            if (q % 8 == 0) {
+                prev_min = quarter_min;
+                quarter_min = 0xffffffffu;
             }
+            quarter_min = std::min(quarter_min, count);
+            if ((int)count != uses[q] || count > prev_min) return bad("incidence counts");
+            std::vector<int> corners;
+            for (uint32_t e = 0; e < count; e++) {
+                if ((int64_t)first + 8 * e >= P.inc_stride) return bad("incidence list past its stride");
+                const uint32_t v = P.tile_inc[b * P.inc_stride + first + 8 * e] / 16, k = v / T, j = v % T;
+                if ((int64_t)j >= ntt || P.lconn[4 * (b * T + j) + k] != q) return bad("incidence entry");
+                corners.push_back((int)v);
+            }
+            std::sort(corners.begin(), corners.end());
+            if (std::unique(corners.begin(), corners.end()) != corners.end()) return bad("repeated incidence entry");
         }
     }
     for (int64_t t = 0; t < nt; t++)
@@ -429,14 +439,14 @@ int nfx_set_mesh(nfx_sim* s, int64_t np, int64_t nt, const double* points, const
     if ((rc = set_device(s)) != NFX_OK) return rc;
     MeshPlan plan;
     std::string err;
-    if (!build_mesh_plan(np, nt, points, tets, s->tile_tets, plan, err)) return fail(NFX_ERR_ARG, err);
+    if (!build_mesh_plan(np, nt, points, tets, s->tile_tets, plan, err, host_threads())) return fail(NFX_ERR_ARG, err);
     CUDA_TRY(cudaStreamSynchronize(s->stream));
     invalidate_graph(s);
     free_mesh(s);
     s->plan = std::move(plan);
     const MeshPlan& P = s->plan;
     auto& A = s->mesh_allocs;
-    int* tb; int* nbg; unsigned* tm; uint2* tn; uchar4* lc; ushort4* ti; float4 *da, *db; float2* dc;
+    int* tb; int* nbg; unsigned* tm; uint2* tn; uchar4* lc; uint4* ti; float4 *da, *db; float2* dc;
     float4 *xh, *xl, *ua, *va, *bbox; float2 *ub, *vb; unsigned long long* fa; double* part; double* tpart;
     const size_t nblk = (size_t)((np + NODE_BLOCK - 1) / NODE_BLOCK);
     const int64_t ns = P.nslots;
@@ -444,7 +454,7 @@ int nfx_set_mesh(nfx_sim* s, int64_t np, int64_t nt, const double* points, const
     if ((rc = dalloc(s, &tb, P.tile_tet_begin.size(), &A)) || (rc = dalloc(s, &nbg, P.tile_node_begin.size(), &A)) ||
         (rc = dalloc(s, &tm, P.tile_meta.size(), &A)) ||
         (rc = dalloc(s, &tn, P.tile_nodes.size() / 2 + ARRAY_PAD, &A)) || (rc = dalloc(s, &lc, ntp, &A)) ||
-        (rc = dalloc(s, &ti, ntp, &A)) ||
+        (rc = dalloc(s, &ti, P.tile_inc.size() / 8, &A)) ||
         (rc = dalloc(s, &da, ntp, &A)) || (rc = dalloc(s, &db, ntp, &A)) || (rc = dalloc(s, &dc, ntp, &A)) ||
         (rc = dalloc(s, &xh, (size_t)np, &A)) || (rc = dalloc(s, &xl, (size_t)np, &A)) || (rc = dalloc(s, &ua, (size_t)np, &A)) ||
         (rc = dalloc(s, &ub, (size_t)np, &A)) || (rc = dalloc(s, &va, (size_t)np, &A)) || (rc = dalloc(s, &vb, (size_t)np, &A)) ||
@@ -468,7 +478,6 @@ int nfx_set_mesh(nfx_sim* s, int64_t np, int64_t nt, const double* points, const
     // zero the padding so bulk copies past a tile's end read defined values
     CUDA_TRY(cudaMemsetAsync(tn, 0, (P.tile_nodes.size() / 2 + ARRAY_PAD) * sizeof(uint2), st));
     CUDA_TRY(cudaMemsetAsync(lc, 0, ntp * sizeof(uchar4), st));
-    CUDA_TRY(cudaMemsetAsync(ti, 0, ntp * sizeof(ushort4), st));
     CUDA_TRY(cudaMemsetAsync(da, 0, ntp * sizeof(float4), st));
     CUDA_TRY(cudaMemsetAsync(db, 0, ntp * sizeof(float4), st));
     CUDA_TRY(cudaMemsetAsync(dc, 0, ntp * sizeof(float2), st));
@@ -502,6 +511,7 @@ int nfx_set_mesh(nfx_sim* s, int64_t np, int64_t nt, const double* points, const
     s->mesh.tile_meta = tm;
     s->mesh.lconn = lc;
     s->mesh.tile_inc = ti;
+    s->mesh.inc_stride = P.inc_stride;
     s->mesh.dmi_a = da;
     s->mesh.dmi_b = db;
     s->mesh.dmi_c = dc;

@@ -150,13 +150,20 @@ int build_plans(nfx_batch* b, const std::vector<int>& which, int tile_tets) {
     const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
     std::vector<std::thread> pool;
     std::atomic<size_t> next{0};
+    // largest meshes first, each with a few threads of its own for its tiles: the time is that of the
+    // largest one
+    std::vector<size_t> turn(owners.size());
+    for (size_t k = 0; k < turn.size(); k++) turn[k] = k;
+    std::stable_sort(turn.begin(), turn.end(), [&](size_t a, size_t c) { return b->cells[owners[a]].nt > b->cells[owners[c]].nt; });
+    const int per_mesh = (int)std::max<unsigned>(1, hw / 4);
     auto work = [&]() {
         for (;;) {
-            const size_t k = next.fetch_add(1);
-            if (k >= owners.size()) return;
+            const size_t at = next.fetch_add(1);
+            if (at >= owners.size()) return;
+            const size_t k = turn[at];
             const CellHost& c = b->cells[owners[k]];
             plans[k] = std::make_shared<MeshPlan>();
-            if (!build_mesh_plan(c.np, c.nt, c.points.data(), c.tets.data(), tile_tets, *plans[k], errs[k]))
+            if (!build_mesh_plan(c.np, c.nt, c.points.data(), c.tets.data(), tile_tets, *plans[k], errs[k], per_mesh))
                 errs[k] = "cell " + std::to_string(owners[k]) + ": " + errs[k];
         }
     };
@@ -326,7 +333,10 @@ int build_device(nfx_batch* b, const std::vector<int>& which, const std::vector<
         std::vector<unsigned> tile_meta(std::max<int64_t>(nti, 1));
         std::vector<uint32_t> tile_nodes(2 * (size_t)ntn);
         std::vector<uint8_t> lconn(4 * ntp, 0);
-        std::vector<uint16_t> tile_inc(4 * ntp, 0);
+        int inc_stride = 8;
+        for (size_t k = 0; k < which.size(); k++)
+            if (bucket[k] == g) inc_stride = std::max(inc_stride, b->cells[which[k]].plan->inc_stride);
+        std::vector<uint16_t> tile_inc((size_t)nti * inc_stride, 0);
         std::vector<float> da(4 * ntp, 0.f), db(4 * ntp, 0.f), dc(2 * ntp, 0.f);
         int64_t tn_pos = 0;
         for (size_t k = 0; k < which.size(); k++) {
@@ -345,7 +355,12 @@ int build_device(nfx_batch* b, const std::vector<int>& which, const std::vector<
             }
             tn_pos += (int64_t)P.tile_nodes.size() / 2;
             std::memcpy(&lconn[4 * c.tet_base], P.lconn.data(), P.lconn.size());
-            std::memcpy(&tile_inc[4 * c.tet_base], P.tile_inc.data(), P.tile_inc.size() * sizeof(uint16_t));
+            if (P.inc_stride == inc_stride)
+                std::memcpy(&tile_inc[c.tile_base * inc_stride], P.tile_inc.data(), P.tile_inc.size() * sizeof(uint16_t));
+            else
+                for (int64_t t = 0; t < P.ntiles; t++)
+                    std::memcpy(&tile_inc[(c.tile_base + t) * inc_stride], &P.tile_inc[t * P.inc_stride],
+                                P.inc_stride * sizeof(uint16_t));
             for (int64_t t = 0; t < P.nslots; t++) {
                 const float* o = &P.dmi[12 * t];
                 const size_t q = (size_t)(c.tet_base + t);
@@ -357,11 +372,11 @@ int build_device(nfx_batch* b, const std::vector<int>& which, const std::vector<
         }
         tile_tet_begin[nti] = (int)nt;
         tile_node_begin[nti] = (int)tn_pos;
-        int* d_ttb; int* d_tnb; unsigned* d_tm; uint2* d_tn; uchar4* d_lc; ushort4* d_ti; float4 *d_da, *d_db;
+        int* d_ttb; int* d_tnb; unsigned* d_tm; uint2* d_tn; uchar4* d_lc; uint4* d_ti; float4 *d_da, *d_db;
         float2* d_dc; int* d_tc;
         float4 *d_pa = nullptr, *d_pb = nullptr; float2 *d_pc = nullptr, *d_fields = nullptr;
         if ((rc = balloc(A, &d_ttb, nti + 1)) || (rc = balloc(A, &d_tnb, nti + 1)) || (rc = balloc(A, &d_tm, nti)) ||
-            (rc = balloc(A, &d_tn, ntn + ARRAY_PAD)) || (rc = balloc(A, &d_lc, ntp)) || (rc = balloc(A, &d_ti, ntp)) ||
+            (rc = balloc(A, &d_tn, ntn + ARRAY_PAD)) || (rc = balloc(A, &d_lc, ntp)) || (rc = balloc(A, &d_ti, tile_inc.size() / 8)) ||
             (rc = balloc(A, &d_da, ntp)) || (rc = balloc(A, &d_db, ntp)) || (rc = balloc(A, &d_dc, ntp)) ||
             (rc = balloc(A, &d_tc, nti)))
             return rc;
@@ -380,7 +395,8 @@ int build_device(nfx_batch* b, const std::vector<int>& which, const std::vector<
         if (ntn > 0)
             BCUDA(cudaMemcpyAsync(d_tn, tile_nodes.data(), tile_nodes.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
         BCUDA(cudaMemcpyAsync(d_lc, lconn.data(), lconn.size(), cudaMemcpyHostToDevice, st));
-        BCUDA(cudaMemcpyAsync(d_ti, tile_inc.data(), tile_inc.size() * sizeof(uint16_t), cudaMemcpyHostToDevice, st));
+        if (nti > 0)
+            BCUDA(cudaMemcpyAsync(d_ti, tile_inc.data(), tile_inc.size() * sizeof(uint16_t), cudaMemcpyHostToDevice, st));
         BCUDA(cudaMemcpyAsync(d_da, da.data(), da.size() * sizeof(float), cudaMemcpyHostToDevice, st));
         BCUDA(cudaMemcpyAsync(d_db, db.data(), db.size() * sizeof(float), cudaMemcpyHostToDevice, st));
         BCUDA(cudaMemcpyAsync(d_dc, dc.data(), dc.size() * sizeof(float), cudaMemcpyHostToDevice, st));
@@ -403,6 +419,7 @@ int build_device(nfx_batch* b, const std::vector<int>& which, const std::vector<
         KM.tile_meta = d_tm;
         KM.lconn = d_lc;
         KM.tile_inc = d_ti;
+        KM.inc_stride = inc_stride;
         KM.dmi_a = d_da;
         KM.dmi_b = d_db;
         KM.dmi_c = d_dc;

@@ -69,8 +69,10 @@ struct MeshPlan {
     std::vector<uint32_t> tile_nodes;      // 2 per node entry: internal node id, (first << 16 | count)
                                            // of its run in the tile's incidence list
     std::vector<uint8_t> lconn;            // 4 * nslots local corner indices
-    std::vector<uint16_t> tile_inc;        // 4 * nslots: per tile, the corners (corner * tile size + local tet)
-                                           // grouped by local node in node order, tet order within
+    int inc_stride = 0;                    // entries per tile of tile_inc, a multiple of 8
+    std::vector<uint16_t> tile_inc;        // ntiles * inc_stride: per tile, the corners of each local node, as byte
+                                           // offsets 16 (corner * tile size + local tet) of the kernels'
+                                           // corner forces; a node's next entry is 8 further on
     std::vector<float> dmi;                // 12 * nslots: Dm^-1 row-major (9), V0, pad, pad
     std::vector<float> Xh, Xl;             // 4 * np: reference position hi / lo parts; Xh.w holds the
                                            // inverse lumped mass of density 1 (VelocityVerlet2)
@@ -81,9 +83,10 @@ struct MeshPlan {
 };
 
 // Builds the plan from the reference's layouts (points SoA 3*np doubles, tets SoA 4*nt).
-// Returns false with a message on invalid input (index out of range, degenerate tetra).
+// Returns false with a message on invalid input (index out of range, degenerate tetra). threads:
+// host threads that may share the work.
 bool build_mesh_plan(int64_t np, int64_t nt, const double* points_soa, const uint32_t* tets_soa, int tile_tets,
-                     MeshPlan& plan, std::string& err);
+                     MeshPlan& plan, std::string& err, int threads = 1);
 
 // ---------------------------------------------------------------------------------------
 // Device views passed to kernels by value.
@@ -96,7 +99,8 @@ struct MeshDev {
     const unsigned* tile_meta; // tetra count | node count << 16
     const uint2* tile_nodes;   // (node id, first << 16 | count)
     const uchar4* lconn;
-    const ushort4* tile_inc;   // four incidence entries per tetra slot of the tile
+    const uint4* tile_inc;     // incidence lists, inc_stride entries per tile, eight to a word
+    int inc_stride;
     const float4* dmi_a;  // Dm^-1 entries 0..3
     const float4* dmi_b;  // Dm^-1 entries 4..7
     const float2* dmi_c;  // Dm^-1 entry 8, V0

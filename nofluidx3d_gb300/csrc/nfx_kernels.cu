@@ -183,32 +183,18 @@ __device__ __forceinline__ float fix_to_float(unsigned long long w) {
 
 // One tile node: sum its corner forces in the tile's fixed incidence order and add the sum to
 // the global accumulator as 64-bit fixed point, so the total does not depend on the order in
-// which tiles finish. Incidence entries are corner-force slots (corner * TILE + local tet). One
-// corner per iteration at the 56-register budget (NFX_FLUSH_UNROLL=4 takes four per iteration,
-// in the same order: faster at 64 registers, 5 % slower at 56). Returns false when a component of
-// the sum exceeds the mesh's per-tile bound fix_max (nothing is added then), which keeps every
-// node's accumulator word within its 64-bit range.
-#ifndef NFX_FLUSH_UNROLL
-#define NFX_FLUSH_UNROLL 1
-#endif
-template <int TILE>
+// which tiles finish. Incidence entries are byte offsets of corner forces, a node's one round of
+// its quarter (eight entries) apart; the plan orders them against bank conflicts. Returns false when
+// a component of the sum exceeds the mesh's per-tile bound fix_max (nothing is added then), which
+// keeps every node's accumulator word within its 64-bit range.
 __device__ __forceinline__ bool node_flush(uint2 node, const unsigned short* inc, const float4* s_cf,
                                            const StateDev& s, long long np, float fix_max) {
     const unsigned first = node.y >> 16, count = node.y & 0xffffu;
     if (count == 0) return true;
     const unsigned short* e = inc + first;
     float fx = 0.f, fy = 0.f, fz = 0.f;
-    unsigned q = 0;
-#if NFX_FLUSH_UNROLL == 4
-    for (; q + 4 <= count; q += 4) {
-        const float4 c0 = s_cf[e[q]], c1 = s_cf[e[q + 1]], c2 = s_cf[e[q + 2]], c3 = s_cf[e[q + 3]];
-        fx = (((fx + c0.x) + c1.x) + c2.x) + c3.x;
-        fy = (((fy + c0.y) + c1.y) + c2.y) + c3.y;
-        fz = (((fz + c0.z) + c1.z) + c2.z) + c3.z;
-    }
-#endif
-    for (; q < count; q++) {
-        const float4 c = s_cf[e[q]];
+    for (unsigned q = 0; q < count; q++) {
+        const float4 c = *reinterpret_cast<const float4*>(reinterpret_cast<const char*>(s_cf) + e[8 * q]);
         fx += c.x;
         fy += c.y;
         fz += c.z;
@@ -218,6 +204,20 @@ __device__ __forceinline__ bool node_flush(uint2 node, const unsigned short* inc
     atomicAdd(s.facc + np + node.x, (unsigned long long)fix_round(fy * FORCE_FIX_SCALE));
     atomicAdd(s.facc + 2 * np + node.x, (unsigned long long)fix_round(fz * FORCE_FIX_SCALE));
     return true;
+}
+
+// The tile's incidence list, inc_stride / 8 words: this thread's word is loaded with the tile's other
+// data (load_incidence) and stored once that is under way (stage_incidence), which also copies the
+// rest where a list is longer than the CTA has threads. A loop over both in one place would hold up
+// the gather behind it for a memory latency (30 % of the pass).
+__device__ __forceinline__ uint4 load_incidence(const MeshDev& m, int b, int j) {
+    const int n = m.inc_stride >> 3;
+    return j < n ? __ldcs(m.tile_inc + (size_t)b * n + j) : make_uint4(0u, 0u, 0u, 0u);
+}
+__device__ __forceinline__ void stage_incidence(uint4* s_inc, uint4 first, const MeshDev& m, int b, int j, int threads) {
+    const int n = m.inc_stride >> 3;
+    if (j < n) s_inc[j] = first;
+    for (int i = j + threads; i < n; i += threads) s_inc[i] = __ldcs(m.tile_inc + (size_t)b * n + i);
 }
 
 __device__ __forceinline__ bool clock_bit(const unsigned* mask, int k) { return (mask[k >> 5] >> (k & 31)) & 1u; }
@@ -389,7 +389,7 @@ __global__ void __launch_bounds__(TILE, 65536 / (TILE * NFX_TET_REGS))
     __shared__ float4 s_ul[NMAX];
 #endif
     __shared__ float4 s_cf[4 * TILE];  // corner forces, slot corner*TILE + local tet
-    __shared__ ushort4 s_inc[TILE];    // the tile's incidence list
+    extern __shared__ uint4 s_inc[];   // the tile's incidence list
 #if NFX_DMI_FROM_X
     __shared__ float4 s_xh[NMAX];
     __shared__ float4 s_xl[NMAX];
@@ -435,7 +435,7 @@ __global__ void __launch_bounds__(TILE, 65536 / (TILE * NFX_TET_REGS))
         pb = __ldcs(s.vp_b + t);
         pc = __ldcs(s.vp_c + t);
     }
-    s_inc[j] = __ldcs(m.tile_inc + t);
+    const uint4 inc0 = load_incidence(m, b, j);
     uint2 node = make_uint2(0u, 0u);
 #if NFX_TILE_REL
     // the tile's first node (every thread loads the same words: one broadcast transaction)
@@ -460,6 +460,7 @@ __global__ void __launch_bounds__(TILE, 65536 / (TILE * NFX_TET_REGS))
 #endif
     }
     const MaterialDev mat = bd.cells[bd.tile_cell ? __ldg(bd.tile_cell + b) : 0].mat;
+    stage_incidence(s_inc, inc0, m, b, j, TILE);
     __syncthreads();
 #if NFX_DMI_FROM_X
     float4 da = make_float4(0.f, 0.f, 0.f, 0.f), db = da;
@@ -474,7 +475,7 @@ __global__ void __launch_bounds__(TILE, 65536 / (TILE * NFX_TET_REGS))
         raise_status(s, tile_cell_status(bd, b), STATUS_INVERTED);
 #endif
     __syncthreads();
-    if (j < nn && !node_flush<TILE>(node, reinterpret_cast<const unsigned short*>(s_inc), s_cf, s, m.np, m.fix_max))
+    if (j < nn && !node_flush(node, reinterpret_cast<const unsigned short*>(s_inc), s_cf, s, m.np, m.fix_max))
         raise_status(s, tile_cell_status(bd, b), STATUS_NONFINITE);
 }
 
@@ -491,7 +492,7 @@ __global__ void __launch_bounds__(TILE) k_si_pass(MeshDev m, StateDev s, BatchDe
     constexpr int NMAX = TILE < TILE_NODES_MAX ? TILE : TILE_NODES_MAX;
     __shared__ float4 s_uh[NMAX], s_ul[NMAX], s_xh[NMAX], s_xl[NMAX];
     __shared__ float4 s_cf[4 * TILE];
-    __shared__ ushort4 s_inc[TILE];
+    extern __shared__ uint4 s_inc[];
     __shared__ SphereIntegralStep s_sp;
     __shared__ double s_red[TILE / 32];
     const int b = blockIdx.x, j = threadIdx.x;
@@ -513,7 +514,7 @@ __global__ void __launch_bounds__(TILE) k_si_pass(MeshDev m, StateDev s, BatchDe
         s_xl[j] = m.Xl[node.x];
     }
     const uchar4 lc = m.lconn[t];
-    if (mode == SI_STEP) s_inc[j] = m.tile_inc[t];
+    if (mode == SI_STEP) stage_incidence(s_inc, load_incidence(m, b, j), m, b, j, TILE);
     const long long time = s.clock->time + (mode == SI_STEP ? t_offset : 0);
     if (j == 0) {
         const double cy = contact_pos(C.c[si], time);
@@ -532,7 +533,7 @@ __global__ void __launch_bounds__(TILE) k_si_pass(MeshDev m, StateDev s, BatchDe
     }
     if (mode != SI_STEP) return;
     __syncthreads();
-    if (j < nn && !node_flush<TILE>(node, reinterpret_cast<const unsigned short*>(s_inc), s_cf, s, m.np, m.fix_max))
+    if (j < nn && !node_flush(node, reinterpret_cast<const unsigned short*>(s_inc), s_cf, s, m.np, m.fix_max))
         raise_status(s, bd.cell_status ? bd.cell_status + cell : nullptr, STATUS_NONFINITE);
 }
 
@@ -944,12 +945,24 @@ __global__ void k_vec_from_user(int np, float4* a, float2* b, int part, const lo
 // ------------------------------------------------------------------------------------------
 // Launchers
 // ------------------------------------------------------------------------------------------
+// Dynamic shared memory of a tile's incidence list: 10 bytes a tetra on the meshes measured, at most
+// 24 (a node in every tetra of its tile), which only with 512-tetra tiles can pass 48 KB a CTA.
+static size_t inc_bytes(const MeshDev& m) { return (size_t)m.inc_stride * sizeof(unsigned short); }
+template <int TILE>
+static cudaError_t allow_inc(const void* kernel, const MeshDev& m) {
+    if (TILE < 512) return cudaSuccess;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)inc_bytes(m));
+}
+
 template <int MODEL, int TILE>
 static cudaError_t launch_tet(const MeshDev& m, const StateDev& s, const BatchDev& b, int t_offset, cudaStream_t st,
                               bool pdl) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)m.ntiles);
     cfg.blockDim = dim3(TILE);
+    cfg.dynamicSmemBytes = inc_bytes(m);
+    cudaError_t e = allow_inc<TILE>((const void*)k_tet_pass<MODEL, TILE>, m);
+    if (e != cudaSuccess) return e;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -987,11 +1000,17 @@ cudaError_t launch_si_pass(const MeshDev& m, const StateDev& s, const BatchDev& 
                           int contact, cudaStream_t st) {
     if (m.ntiles <= 0) return cudaSuccess;
     const int mode = readout ? SI_READOUT : SI_STEP;
+    const size_t inc = inc_bytes(m);
     switch (m.tile_tets) {
-        case 64: k_si_pass<64><<<m.ntiles, 64, 0, st>>>(m, s, b, t_offset, mode, contact); break;
-        case 128: k_si_pass<128><<<m.ntiles, 128, 0, st>>>(m, s, b, t_offset, mode, contact); break;
-        case 256: k_si_pass<256><<<m.ntiles, 256, 0, st>>>(m, s, b, t_offset, mode, contact); break;
-        case 512: k_si_pass<512><<<m.ntiles, 512, 0, st>>>(m, s, b, t_offset, mode, contact); break;
+        case 64: k_si_pass<64><<<m.ntiles, 64, inc, st>>>(m, s, b, t_offset, mode, contact); break;
+        case 128: k_si_pass<128><<<m.ntiles, 128, inc, st>>>(m, s, b, t_offset, mode, contact); break;
+        case 256: k_si_pass<256><<<m.ntiles, 256, inc, st>>>(m, s, b, t_offset, mode, contact); break;
+        case 512: {
+            const cudaError_t e = allow_inc<512>((const void*)k_si_pass<512>, m);
+            if (e != cudaSuccess) return e;
+            k_si_pass<512><<<m.ntiles, 512, inc, st>>>(m, s, b, t_offset, mode, contact);
+            break;
+        }
         default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();

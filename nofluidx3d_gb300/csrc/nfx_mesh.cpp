@@ -11,7 +11,10 @@
 //    the fewest new nodes, so tiles are compact and share few nodes (every node entry of a tile
 //    costs a displacement gather and three accumulator atomics per step). Each tetra's corners
 //    are stored as 8-bit indices into its tile's node list, plus the tile's incidence list
-//    (corners grouped by node) for the fixed-order force sums;
+//    (corners grouped by node) for the fixed-order force sums. Local node numbers and the order of
+//    the sums are chosen so that the warps' shared-memory reads meet few bank conflicts: on the
+//    Kuhn spheres the law's corner reads cost 90 passes a tile instead of 126, the force sums' 99
+//    instead of 173 and their list entries 38 instead of 61 (64, 75 and 30 without any conflict);
 //  * Dm^-1 (inverse of the reference edge matrix [X1-X0, X2-X0, X3-X0]) and the signed
 //    reference volume V0 = det(Dm)/6 (TetraCell.py:33-41) are computed in double and stored
 //    as float;
@@ -19,9 +22,11 @@
 // Corner order within a tetra is the user's, so node 0 of each tetra stays the base node of
 // the reference's elastic kernel (tetra.cl:31-35).
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <numeric>
+#include <thread>
 
 #include "nfx_internal.h"
 
@@ -137,10 +142,161 @@ void grow_tiles(int64_t np, int64_t nt, const uint32_t* T, const std::vector<int
     }
 }
 
+// Shared-memory bank groups. A 16-byte read of a warp is served eight lanes (a quarter) at a time and
+// costs one pass per distinct address that falls on the most used of the eight 16-byte bank groups.
+constexpr int BANK_GROUPS = 8;
+
+// Local numbers for a tile's nodes. rank lists them by falling incidence count; every run of eight in
+// that order is a quarter of a warp in the force sums, and stays one (equal counts end together).
+// Within a quarter the nodes are permuted so that the tetrahedra of a quarter (eight consecutive
+// ones) find their k-th corners in different bank groups: loc[node] % 8 is the group. corner[4 j + k]:
+// node of corner k of tetra j.
+void number_nodes(int cnt, int nn, const uint16_t* corner, const std::vector<uint32_t>& rank, std::vector<uint16_t>& loc,
+                  std::vector<uint16_t>& w) {
+    // w[a * nn + b]: how often a and b are read by the same quarter at the same corner
+    w.assign((size_t)nn * nn, 0);
+    for (int j = 0; j < cnt; j += BANK_GROUPS)
+        for (int k = 0; k < 4; k++) {
+            const int n = std::min(BANK_GROUPS, cnt - j);
+            for (int x = 0; x < n; x++)
+                for (int y = 0; y < x; y++) {
+                    const int a = corner[4 * (j + x) + k], c = corner[4 * (j + y) + k];
+                    if (a == c) continue;
+                    w[(size_t)a * nn + c]++;
+                    w[(size_t)c * nn + a]++;
+                }
+        }
+    std::vector<uint16_t> group[BANK_GROUPS];
+    int cost[BANK_GROUPS][BANK_GROUPS];  // [node of the quarter][group]
+    for (int q = 0; q < nn; q += BANK_GROUPS) {
+        const int n = std::min(BANK_GROUPS, nn - q);
+        for (int x = 0; x < n; x++)
+            for (int g = 0; g < n; g++) {
+                cost[x][g] = 0;
+                for (uint16_t o : group[g]) cost[x][g] += w[(size_t)rank[q + x] * nn + o];
+            }
+        int at[BANK_GROUPS];  // group of each node: in order, then improved by swaps
+        for (int x = 0; x < n; x++) at[x] = x;
+        for (bool better = true; better;) {
+            better = false;
+            for (int x = 0; x < n; x++)
+                for (int y = 0; y < x; y++)
+                    if (cost[x][at[y]] + cost[y][at[x]] < cost[x][at[x]] + cost[y][at[y]]) {
+                        std::swap(at[x], at[y]);
+                        better = true;
+                    }
+        }
+        for (int x = 0; x < n; x++) {
+            loc[rank[q + x]] = (uint16_t)(q + at[x]);
+            group[at[x]].push_back((uint16_t)rank[q + x]);
+        }
+    }
+}
+
+// Runs work(b0, b1) over [0, n) on up to `threads` host threads, at least 4 items each. False when a
+// part ran out of memory (an exception must not leave its thread).
+template <class Work>
+bool in_parallel(int64_t n, int threads, const Work& work) {
+    const int64_t parts = std::max<int64_t>(1, std::min<int64_t>(threads, n / 4));
+    std::atomic<bool> failed{false};
+    auto part = [&](int64_t k) {
+        try {
+            work(n * k / parts, n * (k + 1) / parts);
+        } catch (...) {
+            failed = true;
+        }
+    };
+    std::vector<std::thread> pool;
+    int64_t k = 1;
+    try {
+        for (; k < parts; k++) pool.emplace_back(part, k);
+    } catch (...) {  // no more threads: the parts without one run here
+    }
+    part(0);
+    for (; k < parts; k++) part(k);
+    for (auto& t : pool) t.join();
+    return !failed;
+}
+
+// Order in which the eight nodes of a quarter take their corner forces, one each per round: list[l]
+// holds node l's corner slots (corner * T + tetra, bank group tetra % 8) and is put into that order.
+// Each round matches nodes to different bank groups as far as their remaining corners allow
+// (augmenting paths, the groups in most demand first); what is left over takes the least used.
+void order_corners(std::vector<uint16_t> (&list)[BANK_GROUPS], int n) {
+    int left[BANK_GROUPS][BANK_GROUPS] = {}, next[BANK_GROUPS][BANK_GROUPS], demand[BANK_GROUPS] = {};
+    size_t rounds = 0;
+    std::vector<uint16_t> sorted[BANK_GROUPS];  // each node's slots by bank group; next: the first not yet taken
+    for (int l = 0; l < n; l++) {
+        rounds = std::max(rounds, list[l].size());
+        for (uint16_t v : list[l]) left[l][v % BANK_GROUPS]++;
+        int pos = 0, fill[BANK_GROUPS];
+        for (int g = 0; g < BANK_GROUPS; g++) {
+            next[l][g] = fill[g] = pos;
+            pos += left[l][g];
+            demand[g] += left[l][g];
+        }
+        sorted[l].resize(list[l].size());
+        for (uint16_t v : list[l]) sorted[l][fill[v % BANK_GROUPS]++] = v;
+    }
+    unsigned has[BANK_GROUPS] = {};  // per group: the nodes that still have a corner in it, as bits
+    for (int l = 0; l < n; l++)
+        for (int g = 0; g < BANK_GROUPS; g++) has[g] |= (unsigned)(left[l][g] > 0) << l;
+    int order[BANK_GROUPS];
+    for (int g = 0; g < BANK_GROUPS; g++) order[g] = g;
+    for (size_t r = 0; r < rounds; r++) {
+        int take[BANK_GROUPS], load[BANK_GROUPS] = {};
+        std::fill(take, take + BANK_GROUPS, -1);
+        for (int i = 1; i < BANK_GROUPS; i++)  // nearly sorted from the round before
+            for (int k = i; k > 0 && demand[order[k]] > demand[order[k - 1]]; k--) std::swap(order[k], order[k - 1]);
+        unsigned taken = 0;
+        for (int oi = 0; oi < BANK_GROUPS && demand[order[oi]] > 0; oi++) {
+            const int g0 = order[oi];
+            const unsigned open = has[g0] & ~taken;
+            if (open) {  // a node without a group yet
+                const int l = __builtin_ctz(open);
+                take[l] = g0;
+                taken |= 1u << l;
+                continue;
+            }
+            // match the group to a node all the same, moving other groups' nodes along
+            unsigned seen = 0;
+            auto place = [&](auto&& self, int g) -> bool {
+                for (int l = 0; l < n; l++) {
+                    if (!((has[g] >> l) & 1u) || ((seen >> l) & 1u)) continue;
+                    seen |= 1u << l;
+                    if (take[l] < 0 || self(self, take[l])) {
+                        take[l] = g;
+                        taken |= 1u << l;
+                        return true;
+                    }
+                }
+                return false;
+            };
+            place(place, g0);
+        }
+        for (int l = 0; l < n; l++)
+            if (take[l] >= 0) load[take[l]]++;
+        for (int l = 0; l < n; l++) {
+            if (r >= list[l].size()) continue;
+            if (take[l] < 0) {
+                int best = -1;
+                for (int g = 0; g < BANK_GROUPS; g++)
+                    if (left[l][g] && (best < 0 || load[g] < load[best])) best = g;
+                take[l] = best;
+                load[best]++;
+            }
+            const int g = take[l];
+            list[l][r] = sorted[l][next[l][g]++];
+            if (--left[l][g] == 0) has[g] &= ~(1u << l);
+            demand[g]--;
+        }
+    }
+}
+
 }  // namespace
 
 bool build_mesh_plan(int64_t np, int64_t nt, const double* P, const uint32_t* T, int tile_tets, MeshPlan& plan,
-                     std::string& err) {
+                     std::string& err, int threads) {
     if (tile_tets != 64 && tile_tets != 128 && tile_tets != 256 && tile_tets != 512) {
         err = "tile size must be 64, 128, 256 or 512";
         return false;
@@ -222,71 +378,131 @@ bool build_mesh_plan(int64_t np, int64_t nt, const double* P, const uint32_t* T,
     std::vector<int64_t> tile_end;
     grow_tiles(np, nt, T, order, tile_tets, (int)nodes_max, tile_tets_list, tile_end);
     order.assign(tile_tets_list.begin(), tile_tets_list.end());  // tetrahedra in tile order
-    std::vector<int64_t> slot_user;  // tetra slot -> user tetra (-1: padding)
-    std::vector<uint32_t> ids;
-    ids.reserve(4 * (size_t)tile_tets);
-    int64_t t0 = 0, b = 0;
-    while (t0 < nt) {
-        const int64_t cnt = tile_end[b] - t0;
-        ids.clear();
-        for (int64_t j = 0; j < cnt; j++) {
-            const int64_t ut = order[t0 + j];
-            for (int k = 0; k < 4; k++) ids.push_back((uint32_t)plan.node_int[T[k * nt + ut]]);
-        }
-        std::sort(ids.begin(), ids.end());
-        ids.erase(std::unique(ids.begin(), ids.end()), ids.end());
-        const size_t nn = ids.size();
-        const size_t s0 = (size_t)(b * T_);
-        slot_user.resize(s0 + T_, -1);
-        plan.lconn.resize(4 * (s0 + T_), 0);
-        plan.tile_inc.resize(4 * (s0 + T_), 0);
-        // Local node order: by incidence count, largest first (ties by node index). The thread of
-        // local node q sums its corners in a loop, and a warp runs as many iterations as its
-        // largest count, so grouping similar counts into the same warp saves iterations.
-        std::vector<uint32_t> cnt_by_id(nn, 0);
-        for (int64_t j = 0; j < cnt; j++) {
-            const int64_t ut = order[t0 + j];
-            for (int k = 0; k < 4; k++) {
-                const uint32_t g = (uint32_t)plan.node_int[T[k * nt + ut]];
-                cnt_by_id[std::lower_bound(ids.begin(), ids.end(), g) - ids.begin()]++;
+    const int64_t nti = (int64_t)tile_end.size();
+    std::vector<int64_t> slot_user((size_t)(nti * T_), -1);  // tetra slot -> user tetra (-1: padding)
+    plan.lconn.assign(4 * (size_t)(nti * T_), 0);
+    plan.tile_nodes.assign(2 * (size_t)(nti * NM_), 0u);
+    plan.tile_meta.assign((size_t)nti, 0u);
+    std::vector<std::vector<uint16_t>> inc_of_tile((size_t)nti);
+    // Tiles do not depend on one another: build_tiles makes those of [b0, b1).
+    auto build_tiles = [&](int64_t b0, int64_t b1) {
+        std::vector<uint32_t> ids;
+        ids.reserve(4 * (size_t)tile_tets);
+        std::vector<uint16_t> corner, weights;
+        for (int64_t b = b0; b < b1; b++) {
+            const int64_t t0 = b > 0 ? tile_end[b - 1] : 0;
+            const int64_t cnt = tile_end[b] - t0;
+            ids.clear();
+            for (int64_t j = 0; j < cnt; j++) {
+                const int64_t ut = order[t0 + j];
+                for (int k = 0; k < 4; k++) ids.push_back((uint32_t)plan.node_int[T[k * nt + ut]]);
             }
-        }
-        std::vector<uint32_t> by_count(nn), loc_of(nn);
-        std::iota(by_count.begin(), by_count.end(), 0u);
-        std::stable_sort(by_count.begin(), by_count.end(),
-                         [&](uint32_t a, uint32_t c) { return cnt_by_id[a] > cnt_by_id[c]; });
-        for (size_t q = 0; q < nn; q++) loc_of[by_count[q]] = (uint32_t)q;
-        std::vector<uint32_t> count(nn, 0), first(nn, 0);
-        for (int64_t j = 0; j < cnt; j++) {
-            const int64_t ut = order[t0 + j];
-            slot_user[s0 + j] = ut;
-            for (int k = 0; k < 4; k++) {
-                const uint32_t g = (uint32_t)plan.node_int[T[k * nt + ut]];
-                const uint32_t loc = loc_of[std::lower_bound(ids.begin(), ids.end(), g) - ids.begin()];
-                plan.lconn[4 * (s0 + j) + k] = (uint8_t)loc;
-                count[loc]++;
+            std::sort(ids.begin(), ids.end());
+            ids.erase(std::unique(ids.begin(), ids.end()), ids.end());
+            const size_t nn = ids.size();
+            const size_t s0 = (size_t)(b * T_);
+            // Local node order: by incidence count, largest first (ties by node index). The thread of
+            // local node q sums its corners in a loop, and a warp runs as many iterations as its
+            // largest count, so grouping similar counts into the same warp saves iterations. Eight at
+            // a time they are permuted against bank conflicts (number_nodes).
+            corner.resize(4 * (size_t)cnt);
+            std::vector<uint32_t> cnt_by_id(nn, 0);
+            for (int64_t j = 0; j < cnt; j++)
+                for (int k = 0; k < 4; k++) {
+                    const uint32_t g = (uint32_t)plan.node_int[T[k * nt + order[t0 + j]]];
+                    const uint16_t a = (uint16_t)(std::lower_bound(ids.begin(), ids.end(), g) - ids.begin());
+                    corner[4 * j + k] = a;
+                    cnt_by_id[a]++;
+                }
+            std::vector<uint32_t> by_count(nn);
+            std::iota(by_count.begin(), by_count.end(), 0u);
+            std::stable_sort(by_count.begin(), by_count.end(),
+                             [&](uint32_t a, uint32_t c) { return cnt_by_id[a] > cnt_by_id[c]; });
+            std::vector<uint16_t> loc_of(nn);
+            number_nodes((int)cnt, (int)nn, corner.data(), by_count, loc_of, weights);
+            std::vector<uint32_t> node_at(nn);  // local number -> position in ids
+            for (size_t a = 0; a < nn; a++) node_at[loc_of[a]] = (uint32_t)a;
+            std::vector<uint16_t> slots(4 * (size_t)cnt);  // corner slots by local node, in (tet, corner) order
+            std::vector<uint32_t> begin(nn + 1, 0);
+            for (size_t a = 0; a < nn; a++) begin[loc_of[a] + 1] = cnt_by_id[a];
+            for (size_t q = 0; q < nn; q++) begin[q + 1] += begin[q];
+            std::vector<uint32_t> fill(begin.begin(), begin.end() - 1);
+            for (int64_t j = 0; j < cnt; j++) {
+                slot_user[s0 + j] = order[t0 + j];
+                for (int k = 0; k < 4; k++) {
+                    const uint16_t loc = loc_of[corner[4 * j + k]];
+                    plan.lconn[4 * (s0 + j) + k] = (uint8_t)loc;
+                    slots[fill[loc]++] = (uint16_t)(k * T_ + j);
+                }
             }
-        }
-        // incidence list of the tile: corners grouped by local node, in (tet, corner) order, each
-        // entry the corner's slot in the kernels' corner-major shared array (corner * T + tet)
-        for (size_t q = 1; q < nn; q++) first[q] = first[q - 1] + count[q - 1];
-        std::vector<uint32_t> fill(first);
-        for (int64_t j = 0; j < cnt; j++)
-            for (int k = 0; k < 4; k++) {
-                const uint8_t loc = plan.lconn[4 * (s0 + j) + k];
-                plan.tile_inc[4 * s0 + fill[loc]++] = (uint16_t)(k * T_ + j);
+            // Incidence list of the tile: the local nodes of a quarter side by side, eight entries per
+            // round, a node's entries one round apart; a node with fewer than its quarter's most has
+            // unused entries.
+            std::vector<uint32_t> first(nn);
+            std::vector<uint16_t> inc;
+            for (size_t w = 0; w < nn; w += 4 * BANK_GROUPS) {
+                const int nq = (int)std::min<size_t>(4, (nn - w + BANK_GROUPS - 1) / BANK_GROUPS);
+                std::vector<uint16_t> list[4][BANK_GROUPS];
+                int rounds[4] = {};
+                for (int u = 0; u < nq; u++) {
+                    const size_t q = w + u * BANK_GROUPS;
+                    const int n = (int)std::min<size_t>(BANK_GROUPS, nn - q);
+                    for (int l = 0; l < n; l++) {
+                        list[u][l].assign(slots.begin() + begin[q + l], slots.begin() + begin[q + l + 1]);
+                        rounds[u] = std::max(rounds[u], (int)list[u][l].size());
+                    }
+                    order_corners(list[u], n);
+                }
+                // the quarters of a warp read their lists in step: lay them out so that as few as possible
+                // start in the same bank group
+                int perm[4] = {0, 1, 2, 3}, best[4] = {0, 1, 2, 3}, best_cost = -1;
+                do {
+                    int cost = 0, at[4], pos = (int)(inc.size() / BANK_GROUPS);
+                    for (int u = 0; u < nq; u++) {
+                        at[perm[u]] = pos;
+                        pos += rounds[perm[u]];
+                    }
+                    for (int u = 0; u < nq; u++)
+                        for (int v = 0; v < u; v++)
+                            if ((at[u] - at[v]) % BANK_GROUPS == 0) cost += std::min(rounds[u], rounds[v]);
+                    if (best_cost < 0 || cost < best_cost) {
+                        best_cost = cost;
+                        std::copy(perm, perm + 4, best);
+                    }
+                } while (best_cost > 0 && std::next_permutation(perm, perm + nq));
+                for (int v = 0; v < nq; v++) {
+                    const int u = best[v];
+                    const size_t base = inc.size();
+                    inc.resize(base + (size_t)rounds[u] * BANK_GROUPS, 0);
+                    for (int l = 0; l < BANK_GROUPS && w + u * BANK_GROUPS + l < nn; l++) {
+                        first[w + u * BANK_GROUPS + l] = (uint32_t)(base + l);
+                        for (size_t r = 0; r < list[u][l].size(); r++) inc[base + r * BANK_GROUPS + l] = (uint16_t)(16 * list[u][l][r]);
+                    }
+                }
             }
-        plan.tile_nodes.resize(2 * (size_t)((b + 1) * NM_), 0u);
-        for (size_t q = 0; q < nn; q++) {
-            plan.tile_nodes[2 * (b * NM_ + q)] = ids[by_count[q]];
-            plan.tile_nodes[2 * (b * NM_ + q) + 1] = (first[q] << 16) | count[q];
+            inc_of_tile[b] = std::move(inc);
+            for (size_t q = 0; q < nn; q++) {
+                plan.tile_nodes[2 * (b * NM_ + q)] = ids[node_at[q]];
+                plan.tile_nodes[2 * (b * NM_ + q) + 1] = (first[q] << 16) | (begin[q + 1] - begin[q]);
+            }
+            plan.tile_meta[b] = (uint32_t)cnt | ((uint32_t)nn << 16);
         }
-        plan.tile_meta.push_back((uint32_t)cnt | ((uint32_t)nn << 16));
-        t0 += cnt;
-        b++;
+    };
+    if (!in_parallel(nti, threads, build_tiles)) {
+        err = "out of memory";
+        return false;
     }
+    const int64_t b = nti;
     plan.ntiles = b;
     plan.nslots = b * T_;
+    {
+        // the tiles' incidence lists at one stride, that of the longest
+        size_t longest = BANK_GROUPS;
+        for (const auto& v : inc_of_tile) longest = std::max(longest, v.size());
+        plan.inc_stride = (int)longest;
+        plan.tile_inc.assign((size_t)b * longest, 0);
+        for (int64_t q = 0; q < b; q++) std::copy(inc_of_tile[q].begin(), inc_of_tile[q].end(), &plan.tile_inc[q * longest]);
+    }
     {
         // the most tiles any node appears in sets the per-tile bound of the fixed-point sums
         std::vector<int32_t> tiles_of((size_t)np, 0);
