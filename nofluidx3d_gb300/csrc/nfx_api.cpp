@@ -59,7 +59,8 @@ struct nfx_sim {
     bool cell_dirty = true;
     int nblocks = 0;                 // node blocks
     long long record_every = 0, max_rows = 0, fields_every = 0;
-    long long* d_node_user = nullptr;
+    int* d_node_user = nullptr;
+    int* d_tet_user = nullptr;  // tetra slot -> user tetra, with the viscoplastic state
     double* d_stage = nullptr;
     // Per-step position tables of the contacts, two buffers per contact: a new table goes into
     // the buffer the enqueued steps do not read, and the cell table is repointed in stream order.
@@ -131,6 +132,7 @@ void free_mesh(nfx_sim* s) {
     s->st.clock = keep.clock;
     s->st.force_out = keep.force_out;
     s->d_node_user = nullptr;
+    s->d_tet_user = nullptr;
     s->d_stage = nullptr;
     s->have_mesh = false;
 }
@@ -473,7 +475,7 @@ int nfx_set_mesh(nfx_sim* s, int64_t np, int64_t nt, const double* points, const
         c[2 * t] = o[8];
         c[2 * t + 1] = o[9];
     }
-    std::vector<long long> nu(P.node_user.begin(), P.node_user.end());
+    std::vector<int> nu(P.node_user.begin(), P.node_user.end());
     cudaStream_t st = s->stream;
     // zero the padding so bulk copies past a tile's end read defined values
     CUDA_TRY(cudaMemsetAsync(tn, 0, (P.tile_nodes.size() / 2 + ARRAY_PAD) * sizeof(uint2), st));
@@ -493,7 +495,7 @@ int nfx_set_mesh(nfx_sim* s, int64_t np, int64_t nt, const double* points, const
     CUDA_TRY(cudaMemcpyAsync(xh, P.Xh.data(), P.Xh.size() * sizeof(float), cudaMemcpyHostToDevice, st));
     CUDA_TRY(cudaMemcpyAsync(xl, P.Xl.data(), P.Xl.size() * sizeof(float), cudaMemcpyHostToDevice, st));
     CUDA_TRY(cudaMemcpyAsync(bbox, P.block_box.data(), P.block_box.size() * sizeof(float), cudaMemcpyHostToDevice, st));
-    CUDA_TRY(cudaMemcpyAsync(s->d_node_user, nu.data(), nu.size() * sizeof(long long), cudaMemcpyHostToDevice, st));
+    CUDA_TRY(cudaMemcpyAsync(s->d_node_user, nu.data(), nu.size() * sizeof(int), cudaMemcpyHostToDevice, st));
     for (float4* z : {ua, va}) CUDA_TRY(cudaMemsetAsync(z, 0, (size_t)np * sizeof(float4), st));
     for (float2* z : {ub, vb}) CUDA_TRY(cudaMemsetAsync(z, 0, (size_t)np * sizeof(float2), st));
     CUDA_TRY(cudaMemsetAsync(fa, 0, 3 * (size_t)np * sizeof(unsigned long long), st));
@@ -575,8 +577,12 @@ int nfx_set_viscoplastic(nfx_sim* s, const double* par) {
     const size_t ntp = (size_t)s->plan.nslots + ARRAY_PAD;
     if (!s->st.vp_a) {
         if ((rc = dalloc(s, &s->st.vp_a, ntp, &s->mesh_allocs)) || (rc = dalloc(s, &s->st.vp_b, ntp, &s->mesh_allocs)) ||
-            (rc = dalloc(s, &s->st.vp_c, ntp, &s->mesh_allocs)) || (rc = dalloc(s, &s->st.fields, ntp, &s->mesh_allocs)))
+            (rc = dalloc(s, &s->st.vp_c, ntp, &s->mesh_allocs)) || (rc = dalloc(s, &s->st.fields, ntp, &s->mesh_allocs)) ||
+            (rc = dalloc(s, &s->d_tet_user, (size_t)s->plan.nslots, &s->mesh_allocs)))
             return rc;
+        const std::vector<int> tu(s->plan.tet_user.begin(), s->plan.tet_user.end());
+        CUDA_TRY(cudaMemcpyAsync(s->d_tet_user, tu.data(), tu.size() * sizeof(int), cudaMemcpyHostToDevice, s->stream));
+        CUDA_TRY(cudaStreamSynchronize(s->stream));  // tu goes out of scope
     }
     CUDA_TRY(cudaMemsetAsync(s->st.vp_a, 0, ntp * sizeof(float4), s->stream));
     CUDA_TRY(cudaMemsetAsync(s->st.vp_b, 0, ntp * sizeof(float4), s->stream));
@@ -852,13 +858,10 @@ int nfx_get_tet_field(nfx_sim* s, int which, double* out) {
     }
     int rc;
     if ((rc = set_device(s)) != NFX_OK) return rc;
-    std::vector<float> h(2 * (size_t)ns);
     const float2* src = which == 2 ? s->st.vp_c : s->st.fields;
-    CUDA_TRY(cudaMemcpyAsync(h.data(), src, (size_t)ns * sizeof(float2), cudaMemcpyDeviceToHost, s->stream));
+    CUDA_TRY(launch_field_to_user(ns, s->d_tet_user, src, which == 0 ? 0 : 1, s->d_stage, s->stream));
+    CUDA_TRY(cudaMemcpyAsync(out, s->d_stage, (size_t)nt * sizeof(double), cudaMemcpyDeviceToHost, s->stream));
     CUDA_TRY(cudaStreamSynchronize(s->stream));
-    const int comp = which == 0 ? 0 : 1;
-    for (int64_t t = 0; t < ns; t++)
-        if (s->plan.tet_user[t] >= 0) out[s->plan.tet_user[t]] = (double)h[2 * t + comp];
     return NFX_OK;
 }
 
@@ -873,19 +876,9 @@ int nfx_get_plastic_tensor(nfx_sim* s, double* out) {
     }
     int rc;
     if ((rc = set_device(s)) != NFX_OK) return rc;
-    const int64_t ns = s->plan.nslots;
-    std::vector<float> a(4 * (size_t)ns), b(4 * (size_t)ns), c(2 * (size_t)ns);
-    CUDA_TRY(cudaMemcpyAsync(a.data(), s->st.vp_a, (size_t)ns * sizeof(float4), cudaMemcpyDeviceToHost, s->stream));
-    CUDA_TRY(cudaMemcpyAsync(b.data(), s->st.vp_b, (size_t)ns * sizeof(float4), cudaMemcpyDeviceToHost, s->stream));
-    CUDA_TRY(cudaMemcpyAsync(c.data(), s->st.vp_c, (size_t)ns * sizeof(float2), cudaMemcpyDeviceToHost, s->stream));
+    CUDA_TRY(launch_plastic_to_user(s->plan.nslots, nt, s->st, s->d_tet_user, s->d_stage, s->stream));
+    CUDA_TRY(cudaMemcpyAsync(out, s->d_stage, 9 * (size_t)nt * sizeof(double), cudaMemcpyDeviceToHost, s->stream));
     CUDA_TRY(cudaStreamSynchronize(s->stream));
-    for (int64_t t = 0; t < ns; t++) {
-        const int64_t u = s->plan.tet_user[t];
-        if (u < 0) continue;  // padding slot
-        const float P[9] = {a[4 * t], a[4 * t + 1], a[4 * t + 2], a[4 * t + 3], b[4 * t], b[4 * t + 1],
-                            b[4 * t + 2], b[4 * t + 3], c[2 * t]};
-        for (int k = 0; k < 9; k++) out[k * nt + u] = (double)P[k] + ((k % 4 == 0) ? 1.0 : 0.0);
-    }
     return NFX_OK;
 }
 
@@ -1199,28 +1192,14 @@ int nfx_set_plastic_tensor(nfx_sim* s, const double* in) {
     if (!s->have_mesh) return fail(NFX_ERR_STATE, "no mesh");
     if (s->cell.mat.model != MODEL_VP || !s->st.vp_a)
         return fail(NFX_ERR_STATE, "no viscoplastic material: call nfx_set_viscoplastic first");
-    const int64_t nt = s->plan.nt, ns = s->plan.nslots;
+    const int64_t nt = s->plan.nt;
     for (int64_t i = 0; i < 9 * nt; i++) CHECK_ARG(std::isfinite(in[i]), "non-finite plastic tensor entry");
     int rc;
     if ((rc = set_device(s)) != NFX_OK) return rc;
-    // keep the accumulated strain, replace P = Fp - I
-    std::vector<float> a(4 * (size_t)ns, 0.f), b(4 * (size_t)ns, 0.f), c(2 * (size_t)ns, 0.f);
+    // replaces P = Fp - I, keeps the accumulated strain
+    CUDA_TRY(cudaMemcpyAsync(s->d_stage, in, 9 * (size_t)nt * sizeof(double), cudaMemcpyHostToDevice, s->stream));
+    CUDA_TRY(launch_plastic_from_user(s->plan.nslots, nt, s->st, s->d_tet_user, s->d_stage, s->stream));
     CUDA_TRY(cudaStreamSynchronize(s->stream));
-    CUDA_TRY(cudaMemcpyAsync(c.data(), s->st.vp_c, (size_t)ns * sizeof(float2), cudaMemcpyDeviceToHost, s->stream));
-    CUDA_TRY(cudaStreamSynchronize(s->stream));
-    for (int64_t t = 0; t < ns; t++) {
-        const int64_t u = s->plan.tet_user[t];
-        if (u < 0) continue;
-        float P[9];
-        for (int k = 0; k < 9; k++) P[k] = (float)(in[k * nt + u] - ((k % 4 == 0) ? 1.0 : 0.0));
-        for (int k = 0; k < 4; k++) a[4 * t + k] = P[k];
-        for (int k = 0; k < 4; k++) b[4 * t + k] = P[4 + k];
-        c[2 * t] = P[8];
-    }
-    CUDA_TRY(cudaMemcpyAsync(s->st.vp_a, a.data(), (size_t)ns * sizeof(float4), cudaMemcpyHostToDevice, s->stream));
-    CUDA_TRY(cudaMemcpyAsync(s->st.vp_b, b.data(), (size_t)ns * sizeof(float4), cudaMemcpyHostToDevice, s->stream));
-    CUDA_TRY(cudaMemcpyAsync(s->st.vp_c, c.data(), (size_t)ns * sizeof(float2), cudaMemcpyHostToDevice, s->stream));
-    CUDA_TRY(cudaStreamSynchronize(s->stream));  // the host vectors go out of scope
     return NFX_OK;
 }
 

@@ -91,6 +91,8 @@ struct BatchDevice {
     int nblocks = 0;
     StepClock* d_clock = nullptr;
     unsigned* d_status = nullptr;
+    int* d_node_user = nullptr;  // per node: its index in its cell's user order
+    double* d_stage = nullptr;   // positions of one cell in user order
     cudaGraphExec_t graph = nullptr;
     void release() {
         if (graph) cudaGraphExecDestroy(graph);
@@ -220,6 +222,8 @@ int build_device(nfx_batch* b, const std::vector<int>& which, const std::vector<
     // node arrays and the cell table
     std::vector<float> Xh(4 * (size_t)np, 0.f), Xl(4 * (size_t)np, 0.f), box(8 * (size_t)nblocks, 0.f);
     std::vector<int> block_cell(nblocks);
+    std::vector<int> node_user((size_t)np, 0);
+    int64_t max_np = 0;
     std::vector<CellDev> cells(which.size());
     float fix_max = FORCE_FIX_MAX;
     for (size_t k = 0; k < which.size(); k++) {
@@ -227,6 +231,8 @@ int build_device(nfx_batch* b, const std::vector<int>& which, const std::vector<
         const MeshPlan& P = *c.plan;
         std::memcpy(&Xh[4 * c.node_base], P.Xh.data(), P.Xh.size() * sizeof(float));
         std::memcpy(&Xl[4 * c.node_base], P.Xl.data(), P.Xl.size() * sizeof(float));
+        std::copy(P.node_user.begin(), P.node_user.end(), &node_user[c.node_base]);
+        max_np = std::max(max_np, c.np);
         for (int64_t q = 0; q < c.nblocks; q++) block_cell[c.block_base + q] = (int)k;
         std::memcpy(&box[8 * c.block_base], P.block_box.data(), P.block_box.size() * sizeof(float));
         fix_max = std::min(fix_max, P.fix_max);
@@ -269,8 +275,10 @@ int build_device(nfx_batch* b, const std::vector<int>& which, const std::vector<
         (rc = balloc(A, &d_tpart, ntiles)) || (rc = balloc(A, &d_cells, cells.size())) || (rc = balloc(A, &d_bc, nblocks)) ||
         (rc = balloc(A, &d_cc, cells.size())) || (rc = balloc(A, &d_cst, cells.size())) ||
         (rc = balloc(A, &d_curves, 3 * rows * cells.size())) || (rc = balloc(A, &D.d_clock, 1)) ||
-        (rc = balloc(A, &D.d_status, 1)) || (rc = balloc(A, &d_box, 2 * (size_t)nblocks)))
+        (rc = balloc(A, &D.d_status, 1)) || (rc = balloc(A, &d_box, 2 * (size_t)nblocks)) ||
+        (rc = balloc(A, &D.d_node_user, np)) || (rc = balloc(A, &D.d_stage, 3 * (size_t)max_np)))
         return rc;
+    BCUDA(cudaMemcpyAsync(D.d_node_user, node_user.data(), node_user.size() * sizeof(int), cudaMemcpyHostToDevice, st));
     BCUDA(cudaMemcpyAsync(d_box, box.data(), box.size() * sizeof(float), cudaMemcpyHostToDevice, st));
     BCUDA(cudaMemcpyAsync(d_xh, Xh.data(), Xh.size() * sizeof(float), cudaMemcpyHostToDevice, st));
     BCUDA(cudaMemcpyAsync(d_xl, Xl.data(), Xl.size() * sizeof(float), cudaMemcpyHostToDevice, st));
@@ -522,6 +530,18 @@ int autotune_bucket(nfx_batch* b, int g, const std::vector<int>& members, int& b
         }
     }
     return NFX_OK;
+}
+
+// The node arrays of one cell as a mesh of its own, for the layout conversions.
+void cell_view(const nfx_batch* b, int cell, MeshDev& m, StateDev& st) {
+    const int64_t off = b->cells[cell].node_base;
+    m = b->dev.mesh;
+    st = b->dev.st;
+    m.np = (int)b->cells[cell].np;
+    m.Xh += off;
+    m.Xl += off;
+    st.ua += off;
+    st.ub += off;
 }
 
 // rows produced by node passes at times in [t_begin, t_end] (row r is time r*every)
@@ -873,22 +893,12 @@ int nfx_batch_get_points(nfx_batch* b, int cell, double* out) {
     BARG(out, "null out");
     if (!b->finalized) return bfail(NFX_ERR_STATE, "call nfx_batch_finalize first");
     BCUDA(cudaSetDevice(b->device));
-    const CellHost& c = b->cells[cell];
-    const size_t np = (size_t)c.np;
-    std::vector<float> xh(4 * np), xl(4 * np), ua(4 * np), ub(2 * np);
-    const size_t off = (size_t)c.node_base;
-    const MeshDev& M = b->dev.mesh;
-    BCUDA(cudaMemcpyAsync(xh.data(), M.Xh + off, np * sizeof(float4), cudaMemcpyDeviceToHost, b->stream));
-    BCUDA(cudaMemcpyAsync(xl.data(), M.Xl + off, np * sizeof(float4), cudaMemcpyDeviceToHost, b->stream));
-    BCUDA(cudaMemcpyAsync(ua.data(), b->dev.st.ua + off, np * sizeof(float4), cudaMemcpyDeviceToHost, b->stream));
-    BCUDA(cudaMemcpyAsync(ub.data(), b->dev.st.ub + off, np * sizeof(float2), cudaMemcpyDeviceToHost, b->stream));
+    MeshDev m;
+    StateDev st;
+    cell_view(b, cell, m, st);
+    BCUDA(launch_points_to_user(m, st, b->dev.d_node_user + b->cells[cell].node_base, b->dev.d_stage, b->stream));
+    BCUDA(cudaMemcpyAsync(out, b->dev.d_stage, 3 * (size_t)m.np * sizeof(double), cudaMemcpyDeviceToHost, b->stream));
     BCUDA(cudaStreamSynchronize(b->stream));
-    for (size_t i = 0; i < np; i++) {
-        const int64_t u = c.plan->node_user[i];
-        const float lo[3] = {ua[4 * i + 3], ub[2 * i], ub[2 * i + 1]};
-        for (int d = 0; d < 3; d++)
-            out[d * np + u] = ((double)xh[4 * i + d] + (double)xl[4 * i + d]) + ((double)ua[4 * i + d] + (double)lo[d]);
-    }
     return NFX_OK;
 }
 
@@ -901,28 +911,11 @@ int nfx_batch_set_points(nfx_batch* b, int cell, const double* in) {
     const size_t np = (size_t)c.np;
     for (size_t i = 0; i < 3 * np; i++) BARG(std::isfinite(in[i]), "non-finite position");
     BCUDA(cudaSetDevice(b->device));
-    std::vector<float> xh(4 * np), xl(4 * np), ua(4 * np, 0.f), ub(2 * np, 0.f);
-    const size_t off = (size_t)c.node_base;
-    const MeshDev& M = b->dev.mesh;
-    BCUDA(cudaMemcpyAsync(xh.data(), M.Xh + off, np * sizeof(float4), cudaMemcpyDeviceToHost, b->stream));
-    BCUDA(cudaMemcpyAsync(xl.data(), M.Xl + off, np * sizeof(float4), cudaMemcpyDeviceToHost, b->stream));
-    BCUDA(cudaStreamSynchronize(b->stream));
-    // the displacement x - X as float hi + lo, as the single-cell setter forms it on the device
-    for (size_t i = 0; i < np; i++) {
-        const int64_t u = c.plan->node_user[i];
-        float lo[3];
-        for (int d = 0; d < 3; d++) {
-            const double dx = (in[d * np + u] - (double)xh[4 * i + d]) - (double)xl[4 * i + d];
-            const float h = (float)dx;
-            ua[4 * i + d] = h;
-            lo[d] = (float)(dx - (double)h);
-        }
-        ua[4 * i + 3] = lo[0];
-        ub[2 * i] = lo[1];
-        ub[2 * i + 1] = lo[2];
-    }
-    BCUDA(cudaMemcpyAsync(b->dev.st.ua + off, ua.data(), np * sizeof(float4), cudaMemcpyHostToDevice, b->stream));
-    BCUDA(cudaMemcpyAsync(b->dev.st.ub + off, ub.data(), np * sizeof(float2), cudaMemcpyHostToDevice, b->stream));
+    MeshDev m;
+    StateDev st;
+    cell_view(b, cell, m, st);
+    BCUDA(cudaMemcpyAsync(b->dev.d_stage, in, 3 * np * sizeof(double), cudaMemcpyHostToDevice, b->stream));
+    BCUDA(launch_points_from_user(m, st, b->dev.d_node_user + c.node_base, b->dev.d_stage, b->stream));
     BCUDA(cudaStreamSynchronize(b->stream));
     return NFX_OK;
 }

@@ -241,16 +241,23 @@ cudaError_t launch_si_pass(const MeshDev& m, const StateDev& s, const BatchDev& 
 // q[i] = a[i] / b[i] with the element laws' device divide (self-check of its accuracy).
 cudaError_t launch_divide_check(const float* a, const float* b, float* q, long long n, cudaStream_t stream);
 // Conversions between the user's layout (SoA doubles, user order) and the device state.
-cudaError_t launch_points_to_user(const MeshDev& m, const StateDev& s, const long long* node_user, double* out,
+cudaError_t launch_points_to_user(const MeshDev& m, const StateDev& s, const int* node_user, double* out,
                                   cudaStream_t stream);
-cudaError_t launch_points_from_user(const MeshDev& m, const StateDev& s, const long long* node_user,
+cudaError_t launch_points_from_user(const MeshDev& m, const StateDev& s, const int* node_user,
                                     const double* in, cudaStream_t stream);
 // A node vector stored split over a float4 and a float2 array: part 0 is (a.x, a.y, a.z), part 1
 // is (a.w, b.x, b.y) — the velocity and the previous force of va/vb.
-cudaError_t launch_vec_to_user(const MeshDev& m, const float4* a, const float2* b, int part, const long long* node_user,
+cudaError_t launch_vec_to_user(const MeshDev& m, const float4* a, const float2* b, int part, const int* node_user,
                                double* out, cudaStream_t stream);
-cudaError_t launch_vec_from_user(const MeshDev& m, float4* a, float2* b, int part, const long long* node_user,
+cudaError_t launch_vec_from_user(const MeshDev& m, float4* a, float2* b, int part, const int* node_user,
                                  const double* in, cudaStream_t stream);
-cudaError_t launch_init_vp(const MeshDev& m, const StateDev& s, cudaStream_t stream);
+// Per-tetra state of ns slots between the device and user order (tet_user: slot -> user tetra, -1 for
+// padding): one component of a pair per tetra; Fp, SoA of nt doubles per entry.
+cudaError_t launch_field_to_user(int64_t ns, const int* tet_user, const float2* src, int comp, double* out,
+                                 cudaStream_t stream);
+cudaError_t launch_plastic_to_user(int64_t ns, int64_t nt, const StateDev& s, const int* tet_user, double* out,
+                                   cudaStream_t stream);
+cudaError_t launch_plastic_from_user(int64_t ns, int64_t nt, const StateDev& s, const int* tet_user, const double* in,
+                                     cudaStream_t stream);
 
 }  // namespace nfx

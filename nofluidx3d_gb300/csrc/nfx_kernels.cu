@@ -880,25 +880,25 @@ __global__ void __launch_bounds__(CLOCK_WINDOW) k_advance_time(StepClock* c, lon
 // ------------------------------------------------------------------------------------------
 // Layout conversions (user order, SoA doubles) <-> device state
 // ------------------------------------------------------------------------------------------
-__global__ void k_points_to_user(MeshDev m, StateDev s, const long long* node_user, double* out) {
+__global__ void k_points_to_user(MeshDev m, StateDev s, const int* node_user, double* out) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m.np) return;
-    const long long u = node_user[i];
+    const int u = node_user[i];
     const float4 xh = m.Xh[i], xl = m.Xl[i], uh = s.ua[i];
     const float2 lo = s.ub[i];
     const float4 ul = make_float4(uh.w, lo.x, lo.y, 0.f);
     out[u] = ((double)xh.x + (double)xl.x) + ((double)uh.x + (double)ul.x);
-    out[m.np + u] = ((double)xh.y + (double)xl.y) + ((double)uh.y + (double)ul.y);
+    out[m.np + (long long)u] = ((double)xh.y + (double)xl.y) + ((double)uh.y + (double)ul.y);
     out[2 * (long long)m.np + u] = ((double)xh.z + (double)xl.z) + ((double)uh.z + (double)ul.z);
 }
 
-__global__ void k_points_from_user(MeshDev m, StateDev s, const long long* node_user, const double* in) {
+__global__ void k_points_from_user(MeshDev m, StateDev s, const int* node_user, const double* in) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m.np) return;
-    const long long u = node_user[i];
+    const int u = node_user[i];
     const float4 xh = m.Xh[i], xl = m.Xl[i];
     const double dx = (in[u] - (double)xh.x) - (double)xl.x;
-    const double dy = (in[m.np + u] - (double)xh.y) - (double)xl.y;
+    const double dy = (in[m.np + (long long)u] - (double)xh.y) - (double)xl.y;
     const double dz = (in[2 * (long long)m.np + u] - (double)xh.z) - (double)xl.z;
     const float hx = (float)dx, hy = (float)dy, hz = (float)dz;
     s.ua[i] = make_float4(hx, hy, hz, (float)(dx - hx));
@@ -906,11 +906,11 @@ __global__ void k_points_from_user(MeshDev m, StateDev s, const long long* node_
 }
 
 // part 0: (a.x, a.y, a.z); part 1: (a.w, b.x, b.y)
-__global__ void k_vec_to_user(int np, const float4* a, const float2* b, int part, const long long* node_user,
+__global__ void k_vec_to_user(int np, const float4* a, const float2* b, int part, const int* node_user,
                               double* out) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= np) return;
-    const long long u = node_user[i];
+    const int u = node_user[i];
     const float4 q = a[i];
     float x = q.x, y = q.y, z = q.z;
     if (part == 1) {
@@ -920,16 +920,16 @@ __global__ void k_vec_to_user(int np, const float4* a, const float2* b, int part
         z = r.y;
     }
     out[u] = x;
-    out[np + u] = y;
+    out[np + (long long)u] = y;
     out[2 * (long long)np + u] = z;
 }
 
-__global__ void k_vec_from_user(int np, float4* a, float2* b, int part, const long long* node_user,
+__global__ void k_vec_from_user(int np, float4* a, float2* b, int part, const int* node_user,
                                 const double* in) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= np) return;
-    const long long u = node_user[i];
-    const float x = (float)in[u], y = (float)in[np + u], z = (float)in[2 * (long long)np + u];
+    const int u = node_user[i];
+    const float x = (float)in[u], y = (float)in[np + (long long)u], z = (float)in[2 * (long long)np + u];
     float4 q = a[i];
     if (part == 0) {
         q.x = x;
@@ -940,6 +940,42 @@ __global__ void k_vec_from_user(int np, float4* a, float2* b, int part, const lo
         b[i] = make_float2(y, z);
     }
     a[i] = q;
+}
+
+// One component of a per-tetra pair in user order (tet_user: slot -> user tetra, -1 for padding).
+__global__ void k_field_to_user(int ns, const int* tet_user, const float2* src, int comp, double* out) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= ns) return;
+    const int u = tet_user[t];
+    if (u < 0) return;
+    const float2 v = src[t];
+    out[u] = comp == 0 ? v.x : v.y;
+}
+
+// Fp = I + P in user order, SoA of nt doubles per entry.
+__global__ void k_plastic_to_user(int ns, long long nt, StateDev s, const int* tet_user, double* out) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= ns) return;
+    const int u = tet_user[t];
+    if (u < 0) return;
+    const float4 a = s.vp_a[t], b = s.vp_b[t];
+    const float P[9] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, s.vp_c[t].x};
+#pragma unroll
+    for (int k = 0; k < 9; k++) out[k * nt + u] = (double)P[k] + (k % 4 == 0 ? 1.0 : 0.0);
+}
+
+// P = Fp - I from user order; the accumulated strain stays.
+__global__ void k_plastic_from_user(int ns, long long nt, StateDev s, const int* tet_user, const double* in) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= ns) return;
+    const int u = tet_user[t];
+    if (u < 0) return;
+    float P[9];
+#pragma unroll
+    for (int k = 0; k < 9; k++) P[k] = (float)(in[k * nt + u] - (k % 4 == 0 ? 1.0 : 0.0));
+    s.vp_a[t] = make_float4(P[0], P[1], P[2], P[3]);
+    s.vp_b[t] = make_float4(P[4], P[5], P[6], P[7]);
+    s.vp_c[t].x = P[8];
 }
 
 // ------------------------------------------------------------------------------------------
@@ -1037,7 +1073,7 @@ cudaError_t launch_advance_time(const StateDev& s, long long n, long long fields
     return cudaGetLastError();
 }
 
-cudaError_t launch_points_to_user(const MeshDev& m, const StateDev& s, const long long* node_user, double* out,
+cudaError_t launch_points_to_user(const MeshDev& m, const StateDev& s, const int* node_user, double* out,
                                   cudaStream_t st) {
     k_points_to_user<<<(m.np + 255) / 256, 256, 0, st>>>(m, s, node_user, out);
     return cudaGetLastError();
@@ -1054,19 +1090,37 @@ cudaError_t launch_divide_check(const float* a, const float* b, float* q, long l
     return cudaGetLastError();
 }
 
-cudaError_t launch_points_from_user(const MeshDev& m, const StateDev& s, const long long* node_user,
+cudaError_t launch_points_from_user(const MeshDev& m, const StateDev& s, const int* node_user,
                                     const double* in, cudaStream_t st) {
     k_points_from_user<<<(m.np + 255) / 256, 256, 0, st>>>(m, s, node_user, in);
     return cudaGetLastError();
 }
 
-cudaError_t launch_vec_to_user(const MeshDev& m, const float4* a, const float2* b, int part, const long long* node_user,
+cudaError_t launch_field_to_user(int64_t ns, const int* tet_user, const float2* src, int comp, double* out,
+                                 cudaStream_t st) {
+    k_field_to_user<<<(unsigned)((ns + 255) / 256), 256, 0, st>>>((int)ns, tet_user, src, comp, out);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_plastic_to_user(int64_t ns, int64_t nt, const StateDev& s, const int* tet_user, double* out,
+                                   cudaStream_t st) {
+    k_plastic_to_user<<<(unsigned)((ns + 255) / 256), 256, 0, st>>>((int)ns, nt, s, tet_user, out);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_plastic_from_user(int64_t ns, int64_t nt, const StateDev& s, const int* tet_user, const double* in,
+                                     cudaStream_t st) {
+    k_plastic_from_user<<<(unsigned)((ns + 255) / 256), 256, 0, st>>>((int)ns, nt, s, tet_user, in);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_vec_to_user(const MeshDev& m, const float4* a, const float2* b, int part, const int* node_user,
                                double* out, cudaStream_t st) {
     k_vec_to_user<<<(m.np + 255) / 256, 256, 0, st>>>(m.np, a, b, part, node_user, out);
     return cudaGetLastError();
 }
 
-cudaError_t launch_vec_from_user(const MeshDev& m, float4* a, float2* b, int part, const long long* node_user,
+cudaError_t launch_vec_from_user(const MeshDev& m, float4* a, float2* b, int part, const int* node_user,
                                  const double* in, cudaStream_t st) {
     k_vec_from_user<<<(m.np + 255) / 256, 256, 0, st>>>(m.np, a, b, part, node_user, in);
     return cudaGetLastError();
