@@ -183,9 +183,9 @@ cudaError_t launch_nodes(nfx_sim* s, int k, int mode, int readout_contact, bool 
 }
 
 // The integrated sphere contact's own tile pass, when the cell has one.
-cudaError_t launch_si(nfx_sim* s, int k) {
+cudaError_t launch_si(nfx_sim* s, int k, bool pdl = false) {
     if (s->cell.si_contact < 0) return cudaSuccess;
-    return launch_si_pass(s->mesh, s->st, table_view(s), k, false, -1, s->stream);
+    return launch_si_pass(s->mesh, s->st, table_view(s), k, false, -1, s->stream, pdl);
 }
 
 // Before a readout of contact `contact` between steps: the integrated sphere's tile partials.
@@ -197,7 +197,7 @@ cudaError_t prepare_readout(nfx_sim* s, int contact) {
 int enqueue_steps(nfx_sim* s, int n) {
     for (int k = 0; k < n; k++) {
         CUDA_TRY(launch_elem(s, k, true));                    // programmatic dependent launches
-        CUDA_TRY(launch_si(s, k));
+        CUDA_TRY(launch_si(s, k, true));
         CUDA_TRY(launch_nodes(s, k, NODE_UPDATE, -1, true));
     }
     CUDA_TRY(launch_advance_time(s->st, n, s->fields_every, s->record_every, s->stream));

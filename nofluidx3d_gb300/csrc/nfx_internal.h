@@ -226,7 +226,7 @@ enum NodeMode : int { NODE_UPDATE = 0, NODE_READOUT_ROW = 1, NODE_READOUT_VALUE 
 // Node pass over `nblocks` node blocks. NODE_READOUT_VALUE sums contact `readout_contact`'s force
 // per cell into force_out[cell] without updating the state.
 // pdl: programmatic dependent launch, for the NODE_UPDATE pass of a run of steps only (its
-// predecessor then is an element or integrated-sphere pass, launched in plain stream order).
+// predecessor then is an element pass, or an integrated-sphere pass, which ends after its element pass).
 cudaError_t launch_node_pass(const MeshDev& m, const StateDev& s, const BatchDev& b, int nblocks, int t_offset,
                              int mode, int readout_contact, cudaStream_t stream, bool pdl = false);
 // Advance the clock by n steps (n = 0: refresh the masks only) for the given schedules.
@@ -235,9 +235,10 @@ cudaError_t launch_advance_time(const StateDev& s, long long n, long long fields
 // Integrated sphere contact over all tiles (tiles of cells without one return at once). Inside a
 // step (readout false): its forces join the accumulator and, on record steps, the tile partials
 // of the readout are written. readout true: only the tile partials of contact index `contact` at
-// the current positions, for readouts between steps.
+// the current positions, for readouts between steps. pdl: programmatic dependent launch, directly
+// after the step's element pass only.
 cudaError_t launch_si_pass(const MeshDev& m, const StateDev& s, const BatchDev& b, int t_offset, bool readout,
-                           int contact, cudaStream_t stream);
+                           int contact, cudaStream_t stream, bool pdl = false);
 // q[i] = a[i] / b[i] with the element laws' device divide (self-check of its accuracy).
 cudaError_t launch_divide_check(const float* a, const float* b, float* q, long long n, cudaStream_t stream);
 // Conversions between the user's layout (SoA doubles, user order) and the device state.

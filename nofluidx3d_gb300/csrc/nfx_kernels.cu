@@ -485,7 +485,57 @@ __global__ void __launch_bounds__(TILE, 65536 / (TILE * NFX_TET_REGS))
 // to the force accumulator like the element pass's, and on record steps of that contact the
 // tile's share of the readout (sum of the y forces) goes to tile_partials. SI_READOUT: only the
 // readout shares of contact index `contact` at the current positions (readouts between steps).
+//
+// The density decays as exp(-k (distance - R)), so inside a step a tile is left out when none of its
+// node sums could round to a non-zero fixed-point value: a corner force is at most
+// w exp(-k (d - R)) with w = |det| / 4 <= L^3 / 4 for the diagonal L of the box of the tile's current
+// node positions and d the box's distance from the centre, and a node sums at most TILE of them; below
+// 2^-42 of the sum's unit, half of what rounds to one, every word would receive a zero. Where the
+// readout is due all tiles are evaluated (its shares are not rounded). Bound by latency before: every
+// tile took the gather, 16 shared reads and four exponentials a tetra and the force sums; on the
+// R = 21.3 cell a step of all passes 28.5 -> 20.7 us with the test and the overlap below.
+//
+// Launched as a dependent of the element pass: it reads nothing the element pass writes (the
+// positions are those of the node pass before it, which has completed when the element pass's CTAs
+// release their dependents) and their sums meet in integer atomics, so it runs beside the element
+// pass's last CTAs and only ends after it (the wait at every exit), which the node pass relies on.
 enum SiMode : int { SI_STEP = 0, SI_READOUT = 1 };
+
+// Unsigned integer in the order of the float (NaN beyond the infinities).
+__device__ __forceinline__ unsigned ordered(float x) {
+    const unsigned u = __float_as_uint(x);
+    return u ^ ((unsigned)((int)u >> 31) | 0x80000000u);
+}
+__device__ __forceinline__ float from_ordered(unsigned u) {
+    return __uint_as_float(u ^ ((u & 0x80000000u) ? 0x80000000u : 0xffffffffu));
+}
+
+// Whether the sphere's density is too small for any node sum of a tile to round to a non-zero value (see
+// above). box: per warp the least and greatest ordered coordinates of its nodes.
+template <int TILE>
+__device__ __forceinline__ bool sphere_far(const unsigned (*box)[6], int warps, const SphereIntegralStep& sp) {
+    unsigned lo[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu}, hi[3] = {0u, 0u, 0u};
+    for (int w = 0; w < warps; w++)
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            lo[c] = min(lo[c], box[w][c]);
+            hi[c] = max(hi[c], box[w][3 + c]);
+        }
+    float d2 = 0.f, l2 = 0.f, size = fabsf(sp.cy_hi) + sp.radius + 1.0f;
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        const float a = from_ordered(lo[c]), z = from_ordered(hi[c]), ctr = c == 1 ? sp.cy_hi : 0.f;
+        const float d = fmaxf(fmaxf(a - ctr, ctr - z), 0.f);
+        d2 += d * d;
+        l2 += (z - a) * (z - a);
+        size += fmaxf(fabsf(a), fabsf(z));
+    }
+    // 1e-5 of the coordinates covers the rounding of the positions and of the distances
+    const float gap = sqrtf(d2) - sp.radius - 1e-5f * size;
+    const float log_w = 1.5f * logf(l2) + logf(0.25f * TILE);
+    return sp.k > 0.f && log_w - sp.k * gap < -29.2f;  // 42 ln 2 and a little; false for NaN
+}
+
 template <int TILE>
 __global__ void __launch_bounds__(TILE) k_si_pass(MeshDev m, StateDev s, BatchDev bd, int t_offset, int mode,
                                                   int contact) {
@@ -495,46 +545,77 @@ __global__ void __launch_bounds__(TILE) k_si_pass(MeshDev m, StateDev s, BatchDe
     extern __shared__ uint4 s_inc[];
     __shared__ SphereIntegralStep s_sp;
     __shared__ double s_red[TILE / 32];
+    __shared__ unsigned s_box[NMAX / 32][6];
+    if (threadIdx.x == 0) grid_dep_trigger();
     const int b = blockIdx.x, j = threadIdx.x;
     const int cell = bd.tile_cell ? __ldg(bd.tile_cell + b) : 0;
     const CellDev& C = bd.cells[cell];
     const int si = C.si_contact;
-    if (si < 0 || (mode == SI_READOUT && si != contact)) return;  // uniform over the CTA
+    if (si < 0 || (mode == SI_READOUT && si != contact)) {  // uniform over the CTA
+        grid_dep_wait();
+        return;
+    }
     const int t = b * TILE + j;
     const unsigned meta = __ldg(m.tile_meta + b);
     const int ntt = (int)(meta & 0xffffu), nn = (int)(meta >> 16);
+    const long long time = s.clock->time + (mode == SI_STEP ? t_offset : 0);
+    const bool want_partial =
+        mode == SI_READOUT || (si == C.record_contact && clock_bit(s.clock->record_due, t_offset));
     uint2 node = make_uint2(0u, 0u);
+    float4 uh, xh;
     if (j < NMAX) {
         node = m.tile_nodes[b * NMAX + j];
-        const float4 a = s.ua[node.x];
-        const float2 lo = s.ub[node.x];
-        s_uh[j] = a;
-        s_ul[j] = make_float4(a.w, lo.x, lo.y, 0.f);
-        s_xh[j] = m.Xh[node.x];
-        s_xl[j] = m.Xl[node.x];
+        uh = __ldcg(s.ua + node.x);
+        xh = m.Xh[node.x];
     }
-    const uchar4 lc = m.lconn[t];
-    if (mode == SI_STEP) stage_incidence(s_inc, load_incidence(m, b, j), m, b, j, TILE);
-    const long long time = s.clock->time + (mode == SI_STEP ? t_offset : 0);
     if (j == 0) {
         const double cy = contact_pos(C.c[si], time);
         const float hi = (float)cy;
         s_sp = SphereIntegralStep{hi, (float)(cy - (double)hi), (float)C.c[si].radius, (float)C.c[si].k};
     }
+    if (!want_partial) {  // uniform over the CTA
+        if (j < NMAX) {
+            const float x[3] = {xh.x + uh.x, xh.y + uh.y, xh.z + uh.z};
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                const unsigned v = ordered(x[c]);
+                const unsigned lo = __reduce_min_sync(0xffffffffu, j < nn ? v : 0xffffffffu);
+                const unsigned hi = __reduce_max_sync(0xffffffffu, j < nn ? v : 0u);
+                if ((j & 31) == 0) {
+                    s_box[j >> 5][c] = lo;
+                    s_box[j >> 5][3 + c] = hi;
+                }
+            }
+        }
+        __syncthreads();
+        if (sphere_far<TILE>(s_box, (nn + 31) >> 5, s_sp)) {
+            grid_dep_wait();
+            return;
+        }
+    }
+    if (j < NMAX) {
+        const float2 lo = __ldcg(s.ub + node.x);
+        s_uh[j] = uh;
+        s_ul[j] = make_float4(uh.w, lo.x, lo.y, 0.f);
+        s_xh[j] = xh;
+        s_xl[j] = m.Xl[node.x];
+    }
+    const uchar4 lc = m.lconn[t];
+    if (mode == SI_STEP) stage_incidence(s_inc, load_incidence(m, b, j), m, b, j, TILE);
 #pragma unroll
     for (int a = 0; a < 4; a++) s_cf[a * TILE + j] = make_float4(0.f, 0.f, 0.f, 0.f);
     __syncthreads();
     const float fy = j < ntt ? sphere_integral<TILE>(j, lc, s_uh, s_ul, s_xh, s_xl, s_sp, s_cf) : 0.f;
-    const bool want_partial =
-        mode == SI_READOUT || (si == C.record_contact && clock_bit(s.clock->record_due, t_offset));
     if (want_partial) {  // uniform over the CTA
         const double tot = tile_sum<TILE>(fy, s_red);
         if (j == 0) s.tile_partials[m.tile_base + b] = tot;
     }
-    if (mode != SI_STEP) return;
-    __syncthreads();
-    if (j < nn && !node_flush(node, reinterpret_cast<const unsigned short*>(s_inc), s_cf, s, m.np, m.fix_max))
-        raise_status(s, bd.cell_status ? bd.cell_status + cell : nullptr, STATUS_NONFINITE);
+    if (mode == SI_STEP) {
+        __syncthreads();
+        if (j < nn && !node_flush(node, reinterpret_cast<const unsigned short*>(s_inc), s_cf, s, m.np, m.fix_max))
+            raise_status(s, bd.cell_status ? bd.cell_status + cell : nullptr, STATUS_NONFINITE);
+    }
+    grid_dep_wait();
 }
 
 // ------------------------------------------------------------------------------------------
@@ -1032,24 +1113,35 @@ cudaError_t launch_tet_pass(const MeshDev& m, const StateDev& s, const BatchDev&
     }
 }
 
+template <int TILE>
+static cudaError_t launch_si(const MeshDev& m, const StateDev& s, const BatchDev& b, int t_offset, int mode, int contact,
+                             cudaStream_t st, bool pdl) {
+    const cudaError_t e = allow_inc<TILE>((const void*)k_si_pass<TILE>, m);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)m.ntiles);
+    cfg.blockDim = dim3(TILE);
+    cfg.dynamicSmemBytes = inc_bytes(m);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, k_si_pass<TILE>, m, s, b, t_offset, mode, contact);
+}
+
 cudaError_t launch_si_pass(const MeshDev& m, const StateDev& s, const BatchDev& b, int t_offset, bool readout,
-                          int contact, cudaStream_t st) {
+                           int contact, cudaStream_t st, bool pdl) {
     if (m.ntiles <= 0) return cudaSuccess;
     const int mode = readout ? SI_READOUT : SI_STEP;
-    const size_t inc = inc_bytes(m);
     switch (m.tile_tets) {
-        case 64: k_si_pass<64><<<m.ntiles, 64, inc, st>>>(m, s, b, t_offset, mode, contact); break;
-        case 128: k_si_pass<128><<<m.ntiles, 128, inc, st>>>(m, s, b, t_offset, mode, contact); break;
-        case 256: k_si_pass<256><<<m.ntiles, 256, inc, st>>>(m, s, b, t_offset, mode, contact); break;
-        case 512: {
-            const cudaError_t e = allow_inc<512>((const void*)k_si_pass<512>, m);
-            if (e != cudaSuccess) return e;
-            k_si_pass<512><<<m.ntiles, 512, inc, st>>>(m, s, b, t_offset, mode, contact);
-            break;
-        }
+        case 64: return launch_si<64>(m, s, b, t_offset, mode, contact, st, pdl);
+        case 128: return launch_si<128>(m, s, b, t_offset, mode, contact, st, pdl);
+        case 256: return launch_si<256>(m, s, b, t_offset, mode, contact, st, pdl);
+        case 512: return launch_si<512>(m, s, b, t_offset, mode, contact, st, pdl);
         default: return cudaErrorInvalidValue;
     }
-    return cudaGetLastError();
 }
 
 cudaError_t launch_node_pass(const MeshDev& m, const StateDev& s, const BatchDev& b, int nblocks, int t_offset,
