@@ -80,6 +80,13 @@ struct nfx_sim {
     unsigned* d_status = nullptr;
     StepClock* d_clock = nullptr;
     unsigned* d_counter = nullptr;
+    // runs of steps in one cooperative launch: the barrier's arrival counter, its value after the work
+    // enqueued so far, and the most tiles the current mesh and model may have for its forms (-1: not
+    // looked up)
+    unsigned* d_arrivals = nullptr;
+    unsigned arrivals = 0;
+    int run_tiles[2] = {-1, -1};
+    unsigned long long* d_run_acc = nullptr;  // three accumulators, allocated with the first run of a mesh
     // Page-locked host memory that kernels write small results into: the readout (first word) and,
     // of small meshes, the positions. The result is there when the stream has been waited for, without
     // a copy behind the kernel.
@@ -138,6 +145,7 @@ void free_mesh(nfx_sim* s) {
     s->st.clock = keep.clock;
     s->st.force_out = keep.force_out;
     s->d_node_user = nullptr;
+    s->d_run_acc = nullptr;
     s->d_tet_user = nullptr;
     s->d_stage = nullptr;
     s->have_mesh = false;
@@ -210,6 +218,64 @@ int enqueue_steps(nfx_sim* s, int n) {
     return NFX_OK;
 }
 
+// The barrier's counter back to zero (a run that timed out leaves it anywhere).
+int reset_arrivals(nfx_sim* s) {
+    CUDA_TRY(cudaMemsetAsync(s->d_arrivals, 0, sizeof(unsigned), s->stream));
+    s->arrivals = 0;
+    return NFX_OK;
+}
+
+// Shortest and longest run of steps in one cooperative launch. A run pays a launch, the clearing of its
+// accumulators and the loading of the tiles (about 6 us, a step of the two passes) once.
+constexpr int RUN_STEPS_MIN = 4, RUN_STEPS_MAX = 1024;
+
+// Whether the cell's steps go in cooperative runs (k_run): all its tiles must fit the GPU at once.
+int use_runs(nfx_sim* s, bool& yes) {
+    yes = false;
+    if (s->cell.si_contact >= 0 || !s->plan.all_nodes_used) return NFX_OK;
+    if (s->run_tiles[0] < 0) CUDA_TRY(run_tiles_max(s->mesh, s->cell.mat.model, s->run_tiles));
+    yes = s->mesh.ntiles <= std::max(s->run_tiles[0], s->run_tiles[1]);
+    if (yes && !s->d_run_acc) return dalloc(s, &s->d_run_acc, 9 * (size_t)s->plan.np, &s->mesh_allocs);
+    return NFX_OK;
+}
+
+// Steps from time t on before one that records a row or writes fields (0: that is step t itself).
+long long plain_steps(const nfx_sim* s, long long t, long long most) {
+    long long n = most;
+    if (s->cell.record_contact >= 0 && s->record_every > 0)
+        n = std::min(n, (t + s->record_every - 1) / s->record_every * s->record_every - t);
+    if (s->cell.mat.model == MODEL_VP && s->fields_every > 0)
+        n = std::min(n, (t + s->fields_every) / s->fields_every * s->fields_every - 1 - t);
+    return n;
+}
+
+// n steps: cooperative runs with the two passes for the steps that record between them.
+int run_steps(nfx_sim* s, int64_t n) {
+    for (int64_t done = 0; done < n;) {
+        const long long t = s->time + done;
+        const long long most = std::min<long long>(n - done, RUN_STEPS_MAX);
+        const long long plain = plain_steps(s, t, most);
+        if (plain >= RUN_STEPS_MIN) {
+            CUDA_TRY(cudaMemsetAsync(s->d_run_acc, 0, 9 * (size_t)s->plan.np * sizeof(unsigned long long), s->stream));
+            CUDA_TRY(launch_run(s->mesh, s->st, table_view(s), s->cell.mat.model,
+                                s->mesh.ntiles <= s->run_tiles[0] ? 0 : 1, s->d_arrivals, s->arrivals, s->d_run_acc,
+                                (int)plain, s->stream));
+            s->arrivals += (unsigned)plain * (unsigned)s->mesh.ntiles;
+            CUDA_TRY(launch_advance_time(s->st, plain, s->fields_every, s->record_every, s->stream));
+            done += plain;
+        } else {
+            // up to the next stretch worth a run: the due steps and the few between them
+            long long k = plain + 1;
+            while (k < most && k < GRAPH_STEPS && plain_steps(s, t + k, most - k) < std::min<long long>(RUN_STEPS_MIN, most - k)) k++;
+            k = std::min(k, most);
+            const int rc = enqueue_steps(s, (int)k);
+            if (rc != NFX_OK) return rc;
+            done += k;
+        }
+    }
+    return NFX_OK;
+}
+
 int build_graph(nfx_sim* s) {
     invalidate_graph(s);
     cudaGraph_t g = nullptr;
@@ -231,7 +297,10 @@ int build_graph(nfx_sim* s) {
 // A new material: the captured graph holds the kernel of one material model, so it is rebuilt only
 // when the model changes; parameters travel through the table.
 void set_material(nfx_sim* s, const MaterialDev& m) {
-    if (!s->have_material || s->cell.mat.model != m.model) invalidate_graph(s);
+    if (!s->have_material || s->cell.mat.model != m.model) {
+        invalidate_graph(s);
+        s->run_tiles[0] = -1;
+    }
     s->cell.mat = m;
     s->cell_dirty = true;
     s->have_material = true;
@@ -386,7 +455,7 @@ int nfx_create(int device, nfx_sim** out) {
     e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) { delete s; return fail(NFX_ERR_CUDA, std::string("cudaStreamCreate: ") + cudaGetErrorString(e)); }
     if ((rc = dalloc(s, &s->d_status, 1, nullptr)) != NFX_OK || (rc = dalloc(s, &s->d_clock, 1, nullptr)) != NFX_OK ||
-        (rc = dalloc(s, &s->d_counter, 1, nullptr)) != NFX_OK ||
+        (rc = dalloc(s, &s->d_counter, 1, nullptr)) != NFX_OK || (rc = dalloc(s, &s->d_arrivals, 1, nullptr)) != NFX_OK ||
         (rc = dalloc(s, &s->d_cell, 1, nullptr)) != NFX_OK) {
         nfx_destroy(s);
         return rc;
@@ -399,6 +468,7 @@ int nfx_create(int device, nfx_sim** out) {
     cudaMemsetAsync(s->d_status, 0, sizeof(unsigned), s->stream);
     cudaMemsetAsync(s->d_clock, 0, sizeof(StepClock), s->stream);
     cudaMemsetAsync(s->d_counter, 0, sizeof(unsigned), s->stream);
+    cudaMemsetAsync(s->d_arrivals, 0, sizeof(unsigned), s->stream);
     s->st.status = s->d_status;
     s->st.clock = s->d_clock;
     s->st.force_out = s->h_out;
@@ -438,6 +508,7 @@ int nfx_destroy(nfx_sim* s) {
     if (s->d_status) cudaFree(s->d_status);
     if (s->d_clock) cudaFree(s->d_clock);
     if (s->d_counter) cudaFree(s->d_counter);
+    if (s->d_arrivals) cudaFree(s->d_arrivals);
     if (s->h_out) cudaFreeHost(s->h_out);
     if (s->d_cell) cudaFree(s->d_cell);
     if (s->stream) cudaStreamDestroy(s->stream);
@@ -513,6 +584,7 @@ int nfx_set_mesh(nfx_sim* s, int64_t np, int64_t nt, const double* points, const
     CUDA_TRY(cudaMemsetAsync(s->d_clock, 0, sizeof(StepClock), st));
     CUDA_TRY(launch_advance_time(s->st, 0, s->fields_every, s->record_every, st));
     CUDA_TRY(cudaMemsetAsync(s->d_status, 0, sizeof(unsigned), st));
+    if ((rc = reset_arrivals(s)) != NFX_OK) return rc;
     CUDA_TRY(cudaStreamSynchronize(st));  // host vectors a/b/c/nu go out of scope
     s->mesh.np = (int)np;
     s->mesh.nt = (int)nt;
@@ -540,6 +612,7 @@ int nfx_set_mesh(nfx_sim* s, int64_t np, int64_t nt, const double* points, const
     s->st.partials = part;
     s->st.tile_partials = tpart;
     s->time = 0;
+    s->run_tiles[0] = -1;
     s->rows_written = 0;
     s->nblocks = (int)((np + NODE_BLOCK - 1) / NODE_BLOCK);
     s->cell.fix_a = s->cell.fix_b = -1;
@@ -758,6 +831,12 @@ int nfx_step(nfx_sim* s, int64_t nsteps) {
     if ((rc = upload_cell(s)) != NFX_OK) return rc;
     const long long t_begin = s->time;
     int64_t left = nsteps;
+    bool runs = false;
+    if ((rc = use_runs(s, runs)) != NFX_OK) return rc;
+    if (runs) {
+        if ((rc = run_steps(s, nsteps)) != NFX_OK) return rc;
+        left = 0;
+    }
     while (left >= GRAPH_STEPS) {
         if (!s->graph_valid && (rc = build_graph(s)) != NFX_OK) return rc;
         CUDA_TRY(cudaGraphLaunch(s->graph, s->stream));
@@ -1196,6 +1275,7 @@ int nfx_checkpoint_load(nfx_sim* s, const void* buf, int64_t bytes) {
     if (h.rows > 0) CUDA_TRY(cudaMemcpyAsync(s->d_curve, p, 3 * sizeof(double) * (size_t)h.rows, cudaMemcpyHostToDevice, s->stream));
     CUDA_TRY(cudaMemsetAsync(s->st.facc, 0, 3 * (size_t)s->plan.np * sizeof(unsigned long long), s->stream));
     CUDA_TRY(cudaMemcpyAsync(s->d_status, &h.status, sizeof(unsigned), cudaMemcpyHostToDevice, s->stream));
+    if ((rc = reset_arrivals(s)) != NFX_OK) return rc;
     const long long t = h.time;
     CUDA_TRY(cudaMemcpyAsync(&s->d_clock->time, &t, sizeof(long long), cudaMemcpyHostToDevice, s->stream));
     CUDA_TRY(launch_advance_time(s->st, 0, s->fields_every, s->record_every, s->stream));

@@ -44,7 +44,7 @@ inline float force_fix_bound(int max_tiles) {
 constexpr unsigned STATUS_NONFINITE = 1u;   // a position or force became NaN/Inf
 constexpr unsigned STATUS_INVERTED = 2u;    // an element reached det F <= 0
 constexpr unsigned STATUS_CURVE_FULL = 4u;  // a record row fell outside the curve buffer
-constexpr unsigned STATUS_TIMEOUT = 8u;     // reserved: a bounded device wait gave up (no current kernel waits)
+constexpr unsigned STATUS_TIMEOUT = 8u;     // a grid barrier of a run of steps was not met in time
 
 // Extra zeroed elements after every per-tetra array and the tile node list (slack for loads
 // that run past a tile's last real element).
@@ -79,6 +79,7 @@ struct MeshPlan {
     std::vector<float> block_box;          // 8 per node block of NODE_BLOCK internal nodes: bounding box
                                            // of the reference positions (lo xyz, 0, hi xyz, 0), outward-rounded
     int max_tiles_per_node = 1;            // the most tiles that list any one node
+    bool all_nodes_used = false;           // every node belongs to a tetra
     float fix_max = FORCE_FIX_MAX;         // per-tile fixed-point bound, force_fix_bound(max_tiles_per_node)
 };
 
@@ -232,6 +233,15 @@ cudaError_t launch_node_pass(const MeshDev& m, const StateDev& s, const BatchDev
 // Advance the clock by n steps (n = 0: refresh the masks only) for the given schedules.
 cudaError_t launch_advance_time(const StateDev& s, long long n, long long fields_every, long long record_every,
                                 cudaStream_t stream);
+// Whole runs of steps of a small cell (no tile or block maps) in one cooperative launch: tiles, the most
+// tiles a mesh like m may have for the launch's two forms (0: not this mesh), and nsteps steps from
+// the clock's time in form 0 or 1, none of which may record a row or write fields. count: the grid
+// barrier's arrival counter, base its value at the launch; the launch adds nsteps * ntiles. acc: three
+// accumulators of 3 * np words, all zero at the launch. A barrier that is not met within about a
+// second raises STATUS_TIMEOUT and ends the run.
+cudaError_t run_tiles_max(const MeshDev& m, int model, int (&tiles)[2]);
+cudaError_t launch_run(const MeshDev& m, const StateDev& s, const BatchDev& b, int model, int form, unsigned* count,
+                       unsigned base, unsigned long long* acc, int nsteps, cudaStream_t stream);
 // Integrated sphere contact over all tiles (tiles of cells without one return at once). Inside a
 // step (readout false): its forces join the accumulator and, on record steps, the tile partials
 // of the readout are written. readout true: only the tile partials of contact index `contact` at

@@ -104,13 +104,14 @@ __device__ __forceinline__ bool element_eval(int j, long long t, uchar4 lc, floa
     }
     return element_law<MODEL, TILE>(j, t, d, da, db, dc, pa, pb, pc, s_cf, s, mat, write_fields);
 }
-template <int MODEL, int TILE>
-__device__ __forceinline__ bool element_law(int j, long long t, float (&d)[3][3], float4 da, float4 db, float2 dc,
-                                            float4 pa, float4 pb, float2 pc, float4* s_cf, const StateDev& s,
-                                            const MaterialDev& mat, bool write_fields) {
+// The law of one tetra from its displacement differences: the corner forces f, the viscoplastic
+// state pa, pb, pc moved on by the step, its von Mises stress and pressure. Returns det F - 1.
+template <int MODEL>
+__device__ __forceinline__ float element_forces(float (&d)[3][3], float4 da, float4 db, float2 dc, float4& pa,
+                                                float4& pb, float2& pc, const MaterialDev& mat, float (&f)[4][3],
+                                                float& vm, float& pr) {
     const float Dmi[9] = {da.x, da.y, da.z, da.w, db.x, db.y, db.z, db.w, dc.x};
     const float V0 = dc.y;
-    float f[4][3];
     float jm1;
     if (MODEL == MODEL_MR) {
         jm1 = mr_element(d[0], d[1], d[2], Dmi, V0, mat.mu1, mat.mu2, mat.kappa, f);
@@ -130,14 +131,27 @@ __device__ __forceinline__ bool element_law(int j, long long t, float (&d)[3][3]
         par.hard_exp = mat.hard_exp;
         float P[9] = {pa.x, pa.y, pa.z, pa.w, pb.x, pb.y, pb.z, pb.w, pc.x};
         float eps = pc.y;
-        float dP[9], rate, vm, pr;
+        float dP[9], rate;
         vp_element(d[0], d[1], d[2], Dmi, V0, par, P, eps, dP, rate, f, vm, pr, jm1);
 #pragma unroll
         for (int q = 0; q < 9; q++) P[q] += dP[q];
         eps += rate;
-        __stcs(s.vp_a + t, make_float4(P[0], P[1], P[2], P[3]));
-        __stcs(s.vp_b + t, make_float4(P[4], P[5], P[6], P[7]));
-        __stcs(s.vp_c + t, make_float2(P[8], eps));
+        pa = make_float4(P[0], P[1], P[2], P[3]);
+        pb = make_float4(P[4], P[5], P[6], P[7]);
+        pc = make_float2(P[8], eps);
+    }
+    return jm1;
+}
+template <int MODEL, int TILE>
+__device__ __forceinline__ bool element_law(int j, long long t, float (&d)[3][3], float4 da, float4 db, float2 dc,
+                                            float4 pa, float4 pb, float2 pc, float4* s_cf, const StateDev& s,
+                                            const MaterialDev& mat, bool write_fields) {
+    float f[4][3], vm, pr;
+    const float jm1 = element_forces<MODEL>(d, da, db, dc, pa, pb, pc, mat, f, vm, pr);
+    if (MODEL == MODEL_VP) {
+        __stcs(s.vp_a + t, pa);
+        __stcs(s.vp_b + t, pb);
+        __stcs(s.vp_c + t, pc);
         if (write_fields) __stcs(s.fields + t, make_float2(vm, pr));
     }
 #pragma unroll
@@ -164,10 +178,9 @@ __device__ __forceinline__ long long fix_round(float y) {
 // mantissa (the float conversions, 64- and 32-bit alike, run on the narrow FP64 pipe).
 __device__ __forceinline__ float fix_to_float(unsigned long long w) {
     const long long sw = (long long)w;
-    if (sw == 0) return 0.0f;
     const unsigned sign = sw < 0 ? 0x80000000u : 0u;
     unsigned long long a = sw < 0 ? 0ull - w : w;
-    const int lz = __clzll((long long)a);
+    const int lz = __clzll((long long)a) & 63;
     a <<= lz;  // leading one at bit 63
     unsigned long long m = a >> 40;  // 24 significant bits
     const unsigned long long rem = a & ((1ull << 40) - 1ull), half = 1ull << 39;
@@ -178,7 +191,7 @@ __device__ __forceinline__ float fix_to_float(unsigned long long w) {
         e++;
     }
     const unsigned be = (unsigned)(e - 40 + 127);  // times 2^-40; always a normal float
-    return __uint_as_float(sign | (be << 23) | ((unsigned)m & 0x7FFFFFu));
+    return sw == 0 ? 0.0f : __uint_as_float(sign | (be << 23) | ((unsigned)m & 0x7FFFFFu));
 }
 
 // One tile node: sum its corner forces in the tile's fixed incidence order and add the sum to
@@ -193,6 +206,7 @@ __device__ __forceinline__ bool node_flush(uint2 node, const unsigned short* inc
     if (count == 0) return true;
     const unsigned short* e = inc + first;
     float fx = 0.f, fy = 0.f, fz = 0.f;
+#pragma unroll 4
     for (unsigned q = 0; q < count; q++) {
         const float4 c = *reinterpret_cast<const float4*>(reinterpret_cast<const char*>(s_cf) + e[8 * q]);
         fx += c.x;
@@ -709,10 +723,14 @@ __device__ __forceinline__ ContactForce contact_exact(const ContactDev& c, doubl
         r.hit = false;
         return r;
     }
-    const double kd = c.k * dis;
-    r.fx = kd * (rx / len);
-    r.fy = kd * (ry / len);
-    r.fz = kd * (rz / len);
+    // The three quotients by len from one reciprocal, each corrected by its exact residual
+    // (Markstein), which gives the rounded quotient: a double division is a long chain on this
+    // GPU's narrow FP64 pipe, and the nodes in contact are what a small cell's step waits for.
+    const double kd = c.k * dis, inv = 1.0 / len;
+    const double qx = rx * inv, qy = ry * inv, qz = rz * inv;
+    r.fx = kd * fma(fma(-qx, len, rx), inv, qx);
+    r.fy = kd * fma(fma(-qy, len, ry), inv, qy);
+    r.fz = kd * fma(fma(-qz, len, rz), inv, qz);
     return r;
 }
 
@@ -770,6 +788,45 @@ __device__ __forceinline__ NodeLoad node_load(const MeshDev& m, const StateDev& 
     return r;
 }
 
+// The cell's integrator on node i with total force f: velocity v, previous force (or acceleration) fo
+// and displacement uh + ul moved on by one step.
+__device__ __forceinline__ void node_integrate(const MeshDev& m, const CellDev& C, int i, const float4& f,
+                                               const float4& xh, float3& v, float3& fo, float4& uh, float4& ul) {
+    float3 nf;  // the new previous-force slot
+    if (C.integrator == INTEGRATOR_VV2) {
+        // velocityVerlet2.cl:9-13: v = (v + (a_old + f/m)/2) / (1 + xi/2); a = f/m - xi v;
+        // x += v + a/2; the old-force slot keeps a
+        const float minv = xh.w * C.inv_density;
+        const float c = C.vv2_c, xi = C.vv2_xi;
+        const float fx = f.x * minv, fy = f.y * minv, fz = f.z * minv;
+        v.x = c * (v.x + 0.5f * (fo.x + fx));
+        v.y = c * (v.y + 0.5f * (fo.y + fy));
+        v.z = c * (v.z + 0.5f * (fo.z + fz));
+        const float ax = fx - xi * v.x, ay = fy - xi * v.y, az = fz - xi * v.z;
+        df_add(uh.x, ul.x, v.x + 0.5f * ax);
+        df_add(uh.y, ul.y, v.y + 0.5f * ay);
+        df_add(uh.z, ul.z, v.z + 0.5f * az);
+        nf = make_float3(ax, ay, az);
+    } else {
+        const float vv_a = C.vv_a, vv_hb = C.vv_hb, vv_dm = C.vv_dm;
+        v.x = vv_a * v.x + vv_hb * (f.x + fo.x);
+        v.y = vv_a * v.y + vv_hb * (f.y + fo.y);
+        v.z = vv_a * v.z + vv_hb * (f.z + fo.z);
+        df_add(uh.x, ul.x, vv_dm * v.x + 0.5f * f.x);
+        df_add(uh.y, ul.y, vv_dm * v.y + 0.5f * f.y);
+        df_add(uh.z, ul.z, vv_dm * v.z + 0.5f * f.z);
+        if (i == C.fix_a || i == C.fix_b) {  // VelocityVerlet.cl:17-22: x = z = 0
+            const float4 xp = m.Xh[i], xl = m.Xl[i];
+            uh.x = -xp.x;
+            ul.x = -xl.x;
+            uh.z = -xp.z;
+            ul.z = -xl.z;
+        }
+        nf = make_float3(f.x, f.y, f.z);
+    }
+    fo = nf;
+}
+
 __device__ __forceinline__ double node_finish(const MeshDev& m, const StateDev& s, int i, const WallStep* wall,
                                               const float4* box, const NodeLoad& L, const CellDev& C, int rc,
                                               bool update, unsigned* cstat) {
@@ -795,44 +852,13 @@ __device__ __forceinline__ double node_finish(const MeshDev& m, const StateDev& 
     // velocity and previous force: streamed once per step (evict-first)
     const float4 va = __ldcs(s.va + i);
     const float2 vb = __ldcs(s.vb + i);
-    float3 v = make_float3(va.x, va.y, va.z);
-    float3 nf;  // the new previous-force slot
-    if (C.integrator == INTEGRATOR_VV2) {
-        // velocityVerlet2.cl:9-13: v = (v + (a_old + f/m)/2) / (1 + xi/2); a = f/m - xi v;
-        // x += v + a/2; the old-force slot keeps a
-        const float minv = xh.w * C.inv_density;
-        const float c = C.vv2_c, xi = C.vv2_xi;
-        const float fx = f.x * minv, fy = f.y * minv, fz = f.z * minv;
-        v.x = c * (v.x + 0.5f * (va.w + fx));
-        v.y = c * (v.y + 0.5f * (vb.x + fy));
-        v.z = c * (v.z + 0.5f * (vb.y + fz));
-        const float ax = fx - xi * v.x, ay = fy - xi * v.y, az = fz - xi * v.z;
-        df_add(uh.x, ul.x, v.x + 0.5f * ax);
-        df_add(uh.y, ul.y, v.y + 0.5f * ay);
-        df_add(uh.z, ul.z, v.z + 0.5f * az);
-        nf = make_float3(ax, ay, az);
-    } else {
-        const float vv_a = C.vv_a, vv_hb = C.vv_hb, vv_dm = C.vv_dm;
-        v.x = vv_a * v.x + vv_hb * (f.x + va.w);
-        v.y = vv_a * v.y + vv_hb * (f.y + vb.x);
-        v.z = vv_a * v.z + vv_hb * (f.z + vb.y);
-        df_add(uh.x, ul.x, vv_dm * v.x + 0.5f * f.x);
-        df_add(uh.y, ul.y, vv_dm * v.y + 0.5f * f.y);
-        df_add(uh.z, ul.z, vv_dm * v.z + 0.5f * f.z);
-        if (i == C.fix_a || i == C.fix_b) {  // VelocityVerlet.cl:17-22: x = z = 0
-            const float4 xp = m.Xh[i], xl = m.Xl[i];
-            uh.x = -xp.x;
-            ul.x = -xl.x;
-            uh.z = -xp.z;
-            ul.z = -xl.z;
-        }
-        nf = make_float3(f.x, f.y, f.z);
-    }
+    float3 v = make_float3(va.x, va.y, va.z), fo = make_float3(va.w, vb.x, vb.y);
+    node_integrate(m, C, i, f, xh, v, fo, uh, ul);
     if (!isfinite(uh.x + uh.y + uh.z + v.x + v.y + v.z)) raise_status(s, cstat, STATUS_NONFINITE);
     s.ua[i] = make_float4(uh.x, uh.y, uh.z, ul.x);
     s.ub[i] = make_float2(ul.y, ul.z);
-    __stcs(s.va + i, make_float4(v.x, v.y, v.z, nf.x));
-    __stcs(s.vb + i, make_float2(nf.y, nf.z));
+    __stcs(s.va + i, make_float4(v.x, v.y, v.z, fo.x));
+    __stcs(s.vb + i, make_float2(fo.y, fo.z));
     s.facc[i] = 0ull;
     s.facc[np + i] = 0ull;
     s.facc[2 * np + i] = 0ull;
@@ -938,6 +964,177 @@ __global__ void __launch_bounds__(NODE_BLOCK, NFX_NODE_MIN_BLOCKS) k_node_pass(M
             r[2] = tot;
         }
         bd.cell_counter[cell] = 0u;
+    }
+}
+
+// ------------------------------------------------------------------------------------------
+// Runs of steps of a small cell in one cooperative launch
+// ------------------------------------------------------------------------------------------
+// A cell whose tiles all fit the GPU at once spends its step on latency: of 5.9 us at R = 8 (102 tiles)
+// the two launches' gaps and the reloading of constants take about half. k_run keeps one CTA per
+// tile for the whole run of steps, with the tile's constants, plastic state and list in registers
+// and shared memory, and a thread per tile node with that node's displacement, velocity and force.
+// Every tile that lists a node moves it itself from the same accumulated force, so all hold the
+// same bits, displacements never leave the CTA, and one grid barrier a step is enough: the sums of step
+// k go to buffer k % 3, are read after barrier k, and the buffer that step k + 1 will use is cleared
+// before barrier k by the threads that own its nodes (it was last read before barrier k - 1). The
+// arithmetic is that of the two passes, so the states agree bit for bit. A step at R = 8 under a flat
+// indenter goes from 5.9 to 4.2 us (100 steps and their readout 660 -> 455). Steps that record a force
+// row or write stress fields take the two passes; so do cells with an integrated sphere and meshes
+// with nodes in no tetra.
+constexpr int RUN_TILE = DEFAULT_TILE_TETS;
+// Two forms, by the tiles an SM has to hold: up to four at 128 registers, up to six at 80. Measured, us a
+// step, two passes / four / six (sphere indenter): R = 8 elastic (102 tiles) 7.9 / 4.9 / 5.4, R = 12
+// viscoplastic (338) 9.3 / 6.1 / 6.3, R = 14 (541) 10.2 / 6.4 / 6.4, R = 16 elastic (809) 10.2 / - / 7.1,
+// viscoplastic 11.7 / - / 8.4; under a flat indenter R = 8 5.9 / 4.2. What is left of the 4.2 is the
+// barrier (1.3), the sums' reads (1.2 with the contacts), the force sums (0.6) and the law (0.3).
+constexpr int RUN_PER_SM[2] = {4, 6};
+// Polls after which a barrier gives up (about a second), raises STATUS_TIMEOUT and ends the run.
+constexpr unsigned RUN_SPIN_LIMIT = 1u << 21;
+
+// Waits until every CTA of the launch has arrived (target: the arrival count that makes it so). What a
+// thread wrote before is visible to all after. False when the wait ran out; uniform over the CTA.
+__device__ __forceinline__ bool grid_barrier(unsigned* count, unsigned target, int* s_ok) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
+        unsigned v, polls = 0;
+        bool ok;
+        do {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
+            ok = (int)(v - target) >= 0;
+        } while (!ok && ++polls < RUN_SPIN_LIMIT);
+        *s_ok = ok;
+    }
+    __syncthreads();
+    return *s_ok != 0;
+}
+
+template <int MODEL, int PER_SM>
+__global__ void __launch_bounds__(RUN_TILE, PER_SM) k_run(MeshDev m, StateDev s, BatchDev bd, unsigned* count, unsigned base,
+                                                     unsigned long long* acc, int nsteps) {
+    __shared__ float4 s_v[RUN_TILE];
+    __shared__ float4 s_cf[4 * RUN_TILE];
+    __shared__ float4 s_ref[2];  // displacement of the tile's first node, hi and lo
+    __shared__ WallStep s_wall[MAX_CONTACTS];
+    __shared__ CellDev C;  // the barriers' acquires empty L1: what every step reads stays in shared memory
+    __shared__ long long s_meta[MAX_CONTACTS][2];
+    __shared__ int s_ok;
+    extern __shared__ uint4 s_inc[];
+    const int b = blockIdx.x, j = threadIdx.x;
+    static_assert(sizeof(CellDev) % 4 == 0, "copied by words");
+    for (int w = j; w < (int)(sizeof(CellDev) / 4); w += RUN_TILE)
+        reinterpret_cast<unsigned*>(&C)[w] = reinterpret_cast<const unsigned*>(bd.cells)[w];
+    __syncthreads();
+    if (j < C.n_contacts) {
+        s_meta[j][0] = C.c[j].meta[0];
+        s_meta[j][1] = C.c[j].meta[1];
+        C.c[j].meta = s_meta[j];
+    }
+    const long long t0 = s.clock->time, np = m.np;
+    // the thread's tetra
+    const int t = b * RUN_TILE + j;
+    const unsigned meta = __ldg(m.tile_meta + b);
+    const int ntt = (int)(meta & 0xffffu), nn = (int)(meta >> 16);
+    const uchar4 lc = m.lconn[t];
+    const float4 da = m.dmi_a[t], db = m.dmi_b[t];
+    const float2 dc = m.dmi_c[t];
+    float4 pa = make_float4(0.f, 0.f, 0.f, 0.f), pb = pa;
+    float2 pc = make_float2(0.f, 0.f);
+    if (MODEL == MODEL_VP) {
+        pa = s.vp_a[t];
+        pb = s.vp_b[t];
+        pc = s.vp_c[t];
+    }
+    stage_incidence(s_inc, load_incidence(m, b, j), m, b, j, RUN_TILE);
+    // the thread's tile node
+    const uint2 node = m.tile_nodes[t];
+    const int i = (int)node.x;
+    float4 xh = make_float4(0.f, 0.f, 0.f, 0.f), xl = xh, uh = xh, ul = xh;
+    float3 v = make_float3(0.f, 0.f, 0.f), fo = v;
+    if (j < nn) {
+        xh = m.Xh[i];
+        xl = m.Xl[i];
+        const float4 a = s.ua[i], va = s.va[i];
+        const float2 lo = s.ub[i], vb = s.vb[i];
+        uh = make_float4(a.x, a.y, a.z, 0.f);
+        ul = make_float4(a.w, lo.x, lo.y, 0.f);
+        v = make_float3(va.x, va.y, va.z);
+        fo = make_float3(va.w, vb.x, vb.y);
+    }
+    // the accumulator words the thread clears
+    const int own = ((j >> 5) * (int)gridDim.x + b) * 32 + (j & 31);
+    StateDev sums = s;  // node_flush adds to sums.facc, the buffer of the step
+    sums.facc = acc;
+    unsigned long long *next = acc + 3 * np, *after = acc + 6 * np;  // those of the next two steps
+    unsigned target = base;
+    __syncthreads();
+    for (int k = 0; k < nsteps; k++) {
+        // element pass
+        if (j == 0) {
+            s_ref[0] = uh;
+            s_ref[1] = ul;
+        }
+        __syncthreads();
+        if (j < nn) {
+            const float4 ar = s_ref[0], lr = s_ref[1];
+            s_v[j] = make_float4((uh.x - ar.x) + (ul.x - lr.x), (uh.y - ar.y) + (ul.y - lr.y), (uh.z - ar.z) + (ul.z - lr.z), 0.f);
+        }
+        __syncthreads();
+        if (j < ntt) {
+            const float4 v0 = s_v[lc.x], v1 = s_v[lc.y], v2 = s_v[lc.z], v3 = s_v[lc.w];
+            float d[3][3] = {{v1.x - v0.x, v1.y - v0.y, v1.z - v0.z},
+                             {v2.x - v0.x, v2.y - v0.y, v2.z - v0.z},
+                             {v3.x - v0.x, v3.y - v0.y, v3.z - v0.z}};
+            float f[4][3], vm, pr;
+            const float jm1 = element_forces<MODEL>(d, da, db, dc, pa, pb, pc, C.mat, f, vm, pr);
+#pragma unroll
+            for (int q = 0; q < 4; q++) s_cf[q * RUN_TILE + j] = make_float4(f[q][0], f[q][1], f[q][2], 0.f);
+            if (!(jm1 > -1.0f)) raise_status(s, nullptr, STATUS_INVERTED);
+        }
+        if (own < m.np) {
+            __stcg(next + own, 0ull);
+            __stcg(next + own + np, 0ull);
+            __stcg(next + own + 2 * np, 0ull);
+        }
+        __syncthreads();
+        if (j < nn && !node_flush(node, reinterpret_cast<const unsigned short*>(s_inc), s_cf, sums, np, m.fix_max))
+            raise_status(s, nullptr, STATUS_NONFINITE);
+        const int c0 = j - (RUN_TILE - 32);  // the last warp has the fewest nodes to sum: the contacts' positions
+        if (c0 >= 0 && c0 < C.n_contacts) {
+            const double w = contact_pos(C.c[c0], t0 + k);
+            s_wall[c0] = WallStep{w, (float)w, (float)C.c[c0].radius};
+        }
+        target += gridDim.x;
+        if (!grid_barrier(count, target, &s_ok)) break;
+        // node pass
+        if (j < nn) {
+            const unsigned long long* fa = sums.facc + i;
+            const unsigned long long f0 = __ldcg(fa), f1 = __ldcg(fa + np), f2 = __ldcg(fa + 2 * np);
+            float4 f = make_float4(fix_to_float(f0), fix_to_float(f1), fix_to_float(f2), 0.f);
+            for (int c = 0; c < C.n_contacts; c++) {
+                double fy;
+                contact_force(C.c[c], s_wall[c], xh, &xl, uh, ul, f, fy);
+            }
+            node_integrate(m, C, i, f, xh, v, fo, uh, ul);
+            if (!isfinite(uh.x + uh.y + uh.z + v.x + v.y + v.z)) raise_status(s, nullptr, STATUS_NONFINITE);
+        }
+        unsigned long long* const done = sums.facc;
+        sums.facc = next;
+        next = after;
+        after = done;
+    }
+    if (j == 0 && !s_ok) raise_status(s, nullptr, STATUS_TIMEOUT);
+    if (j < nn) {  // the same values from every tile that lists the node
+        s.ua[i] = make_float4(uh.x, uh.y, uh.z, ul.x);
+        s.ub[i] = make_float2(ul.y, ul.z);
+        s.va[i] = make_float4(v.x, v.y, v.z, fo.x);
+        s.vb[i] = make_float2(fo.y, fo.z);
+    }
+    if (MODEL == MODEL_VP && j < ntt) {
+        s.vp_a[t] = pa;
+        s.vp_b[t] = pb;
+        s.vp_c[t] = pc;
     }
 }
 
@@ -1129,6 +1326,60 @@ static cudaError_t launch_si(const MeshDev& m, const StateDev& s, const BatchDev
     cfg.attrs = attr;
     cfg.numAttrs = pdl ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, k_si_pass<TILE>, m, s, b, t_offset, mode, contact);
+}
+
+template <int MODEL>
+static cudaError_t run_capacity(const MeshDev& m, int (&tiles)[2]) {
+    int dev = 0, sms = 0, coop = 0, per_sm[2] = {0, 0};
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+    if (e == cudaSuccess)
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[0], k_run<MODEL, RUN_PER_SM[0]>, RUN_TILE, inc_bytes(m));
+    if (e == cudaSuccess)
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[1], k_run<MODEL, RUN_PER_SM[1]>, RUN_TILE, inc_bytes(m));
+    for (int k = 0; k < 2; k++) tiles[k] = e == cudaSuccess && coop ? sms * per_sm[k] : 0;
+    return e;
+}
+
+cudaError_t run_tiles_max(const MeshDev& m, int model, int (&tiles)[2]) {
+    tiles[0] = tiles[1] = 0;
+    if (m.tile_tets != RUN_TILE || (m.np + 31) / 32 > (RUN_TILE / 32) * m.ntiles) return cudaSuccess;
+    switch (model) {
+        case MODEL_MR: return run_capacity<MODEL_MR>(m, tiles);
+        case MODEL_SVK: return run_capacity<MODEL_SVK>(m, tiles);
+        case MODEL_SVKK: return run_capacity<MODEL_SVKK>(m, tiles);
+        case MODEL_VP: return run_capacity<MODEL_VP>(m, tiles);
+        default: return cudaErrorInvalidValue;
+    }
+}
+
+template <int MODEL>
+static cudaError_t launch_run_model(const MeshDev& m, const StateDev& s, const BatchDev& b, int form, unsigned* count,
+                                    unsigned base, unsigned long long* acc, int nsteps, cudaStream_t st) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)m.ntiles);
+    cfg.blockDim = dim3(RUN_TILE);
+    cfg.dynamicSmemBytes = inc_bytes(m);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return form == 0 ? cudaLaunchKernelEx(&cfg, k_run<MODEL, RUN_PER_SM[0]>, m, s, b, count, base, acc, nsteps)
+                     : cudaLaunchKernelEx(&cfg, k_run<MODEL, RUN_PER_SM[1]>, m, s, b, count, base, acc, nsteps);
+}
+
+cudaError_t launch_run(const MeshDev& m, const StateDev& s, const BatchDev& b, int model, int form, unsigned* count,
+                       unsigned base, unsigned long long* acc, int nsteps, cudaStream_t st) {
+    switch (model) {
+        case MODEL_MR: return launch_run_model<MODEL_MR>(m, s, b, form, count, base, acc, nsteps, st);
+        case MODEL_SVK: return launch_run_model<MODEL_SVK>(m, s, b, form, count, base, acc, nsteps, st);
+        case MODEL_SVKK: return launch_run_model<MODEL_SVKK>(m, s, b, form, count, base, acc, nsteps, st);
+        case MODEL_VP: return launch_run_model<MODEL_VP>(m, s, b, form, count, base, acc, nsteps, st);
+        default: return cudaErrorInvalidValue;
+    }
 }
 
 cudaError_t launch_si_pass(const MeshDev& m, const StateDev& s, const BatchDev& b, int t_offset, bool readout,

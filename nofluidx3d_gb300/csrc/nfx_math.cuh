@@ -89,14 +89,33 @@ NFX_HD Mat3 disp_grad(const float d1[3], const float d2[3], const float d3[3], c
     return H;
 }
 
-// det(I + H) - 1 = tr H + i2(H) + det H
+// Rounded product and fused a b + c, written out where a product serves several sums: left to the
+// compiler, the sum that it is fused into depends on the kernel around, and the element pass and the
+// runs of steps then differ by an ulp now and then.
+NFX_HD float mul_(float a, float b) {
+#if defined(__CUDA_ARCH__)
+    return __fmul_rn(a, b);
+#else
+    return a * b;
+#endif
+}
+NFX_HD float fma_(float a, float b, float c) {
+#if defined(__CUDA_ARCH__)
+    return fmaf(a, b, c);
+#else
+    return a * b + c;
+#endif
+}
+
+// det(I + H) - 1 = tr H + i2(H) + det H. The rounded products are those that adj_1p(H) needs too.
 NFX_HD float det1p_minus1(const Mat3& H) {
     const float* h = H.m;
     const float t = h[0] + h[4] + h[8];
-    const float i2 = (h[0] * h[4] - h[1] * h[3]) + (h[4] * h[8] - h[5] * h[7]) + (h[0] * h[8] - h[2] * h[6]);
-    const float d = h[0] * (h[4] * h[8] - h[5] * h[7]) - h[1] * (h[3] * h[8] - h[5] * h[6]) +
-                    h[2] * (h[3] * h[7] - h[4] * h[6]);
-    return t + (i2 + d);
+    const float c0 = fma_(h[4], h[8], -mul_(h[5], h[7]));
+    const float c1 = fma_(-h[3], h[8], mul_(h[5], h[6]));
+    const float c2 = fma_(-h[4], h[6], mul_(h[3], h[7]));
+    const float i2 = (fma_(h[0], h[4], -mul_(h[1], h[3])) + c0) + fma_(h[0], h[8], -mul_(h[2], h[6]));
+    return t + (i2 + fma_(h[0], c0, fma_(h[1], c1, mul_(h[2], c2))));
 }
 
 // E = B - I = H + H^T + H H^T for F = I + H, B = F F^T
@@ -191,15 +210,15 @@ NFX_HD Mat3 adj_1p(const Mat3& H) {
     const float d = H.m[3], e = 1.0f + H.m[4], f = H.m[5];
     const float g = H.m[6], h = H.m[7], i = 1.0f + H.m[8];
     Mat3 A;
-    A.m[0] = e * i - f * h;
-    A.m[1] = c * h - b * i;
-    A.m[2] = b * f - c * e;
-    A.m[3] = f * g - d * i;
-    A.m[4] = a * i - c * g;
-    A.m[5] = c * d - a * f;
-    A.m[6] = d * h - e * g;
-    A.m[7] = b * g - a * h;
-    A.m[8] = a * e - b * d;
+    A.m[0] = fma_(e, i, -mul_(f, h));
+    A.m[1] = fma_(c, h, -mul_(b, i));
+    A.m[2] = fma_(b, f, -mul_(c, e));
+    A.m[3] = fma_(-d, i, mul_(f, g));
+    A.m[4] = fma_(a, i, -mul_(c, g));
+    A.m[5] = fma_(c, d, -mul_(a, f));
+    A.m[6] = fma_(-e, g, mul_(d, h));
+    A.m[7] = fma_(b, g, -mul_(a, h));
+    A.m[8] = fma_(a, e, -mul_(b, d));
     return A;
 }
 

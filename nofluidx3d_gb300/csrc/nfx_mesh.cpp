@@ -511,6 +511,7 @@ bool build_mesh_plan(int64_t np, int64_t nt, const double* P, const uint32_t* T,
             for (int64_t e = 0; e < nn; e++) tiles_of[plan.tile_nodes[2 * (q * NM_ + e)]]++;
         }
         plan.max_tiles_per_node = std::max(1, *std::max_element(tiles_of.begin(), tiles_of.end()));
+        plan.all_nodes_used = *std::min_element(tiles_of.begin(), tiles_of.end()) > 0;
         plan.fix_max = force_fix_bound(plan.max_tiles_per_node);
     }
     plan.tet_user = std::move(slot_user);
