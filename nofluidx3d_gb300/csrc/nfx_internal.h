@@ -1,6 +1,7 @@
 // Internal data structures shared by the host runtime (nfx_api.cpp, nfx_mesh.cpp) and the
 // kernels (nfx_kernels.cu). Not part of the C ABI.
 #pragma once
+#include <functional>
 #include <cuda_runtime.h>
 #include <nvtx3/nvToolsExt.h>
 
@@ -82,6 +83,10 @@ struct MeshPlan {
     bool all_nodes_used = false;           // every node belongs to a tetra
     float fix_max = FORCE_FIX_MAX;         // per-tile fixed-point bound, force_fix_bound(max_tiles_per_node)
 };
+
+// Runs work(b0, b1) over [0, n) on up to `threads` host threads, at least 4 items each. False when a
+// part ran out of memory (an exception must not leave its thread).
+bool in_parallel(int64_t n, int threads, const std::function<void(int64_t, int64_t)>& work);
 
 // Builds the plan from the reference's layouts (points SoA 3*np doubles, tets SoA 4*nt).
 // Returns false with a message on invalid input (index out of range, degenerate tetra). threads:

@@ -25,6 +25,7 @@
 #include <atomic>
 #include <cmath>
 #include <cstring>
+#include <functional>
 #include <numeric>
 #include <thread>
 
@@ -166,14 +167,15 @@ void number_nodes(int cnt, int nn, const uint16_t* corner, const std::vector<uin
                     w[(size_t)c * nn + a]++;
                 }
         }
-    std::vector<uint16_t> group[BANK_GROUPS];
+    uint16_t group[BANK_GROUPS][TILE_NODES_MAX / BANK_GROUPS];  // the nodes of each group so far
+    int held[BANK_GROUPS] = {};
     int cost[BANK_GROUPS][BANK_GROUPS];  // [node of the quarter][group]
     for (int q = 0; q < nn; q += BANK_GROUPS) {
         const int n = std::min(BANK_GROUPS, nn - q);
         for (int x = 0; x < n; x++)
             for (int g = 0; g < n; g++) {
                 cost[x][g] = 0;
-                for (uint16_t o : group[g]) cost[x][g] += w[(size_t)rank[q + x] * nn + o];
+                for (int o = 0; o < held[g]; o++) cost[x][g] += w[(size_t)rank[q + x] * nn + group[g][o]];
             }
         int at[BANK_GROUPS];  // group of each node: in order, then improved by swaps
         for (int x = 0; x < n; x++) at[x] = x;
@@ -188,15 +190,89 @@ void number_nodes(int cnt, int nn, const uint16_t* corner, const std::vector<uin
         }
         for (int x = 0; x < n; x++) {
             loc[rank[q + x]] = (uint16_t)(q + at[x]);
-            group[at[x]].push_back((uint16_t)rank[q + x]);
+            group[at[x]][held[at[x]]++] = (uint16_t)rank[q + x];
         }
     }
 }
 
-// Runs work(b0, b1) over [0, n) on up to `threads` host threads, at least 4 items each. False when a
-// part ran out of memory (an exception must not leave its thread).
-template <class Work>
-bool in_parallel(int64_t n, int threads, const Work& work) {
+// Order in which the n <= 8 nodes of a quarter take their corner forces, one each per round: slots[begin[l]
+// .. begin[l + 1]) are node l's corner slots (corner * T + tetra, bank group tetra % 8), put into that order.
+// Each round matches nodes to different bank groups as far as their remaining corners allow
+// (augmenting paths, the groups in most demand first); what is left over takes the least used.
+void order_corners(uint16_t* slots, const uint32_t* begin, int n, std::vector<uint16_t>& sorted) {
+    int left[BANK_GROUPS][BANK_GROUPS] = {}, next[BANK_GROUPS][BANK_GROUPS], demand[BANK_GROUPS] = {};
+    uint32_t rounds = 0;
+    sorted.resize(begin[n] - begin[0]);  // each node's slots by bank group; next: the first not yet taken
+    for (int l = 0; l < n; l++) {
+        rounds = std::max(rounds, begin[l + 1] - begin[l]);
+        for (uint32_t i = begin[l]; i < begin[l + 1]; i++) left[l][slots[i] % BANK_GROUPS]++;
+        int pos = (int)(begin[l] - begin[0]), fill[BANK_GROUPS];
+        for (int g = 0; g < BANK_GROUPS; g++) {
+            next[l][g] = fill[g] = pos;
+            pos += left[l][g];
+            demand[g] += left[l][g];
+        }
+        for (uint32_t i = begin[l]; i < begin[l + 1]; i++) sorted[fill[slots[i] % BANK_GROUPS]++] = slots[i];
+    }
+    unsigned has[BANK_GROUPS] = {};  // per group: the nodes that still have a corner in it, as bits
+    for (int l = 0; l < n; l++)
+        for (int g = 0; g < BANK_GROUPS; g++) has[g] |= (unsigned)(left[l][g] > 0) << l;
+    int order[BANK_GROUPS];
+    for (int g = 0; g < BANK_GROUPS; g++) order[g] = g;
+    for (uint32_t r = 0; r < rounds; r++) {
+        int take[BANK_GROUPS], load[BANK_GROUPS] = {};
+        std::fill(take, take + BANK_GROUPS, -1);
+        for (int i = 1; i < BANK_GROUPS; i++)  // nearly sorted from the round before
+            for (int k = i; k > 0 && demand[order[k]] > demand[order[k - 1]]; k--) std::swap(order[k], order[k - 1]);
+        unsigned taken = 0, open_nodes = 0;
+        for (int g = 0; g < BANK_GROUPS; g++) open_nodes |= has[g];
+        for (int oi = 0; oi < BANK_GROUPS && demand[order[oi]] > 0 && taken != open_nodes; oi++) {
+            const int g0 = order[oi];
+            const unsigned open = has[g0] & ~taken;
+            if (open) {  // a node without a group yet
+                const int l = __builtin_ctz(open);
+                take[l] = g0;
+                taken |= 1u << l;
+                continue;
+            }
+            // match the group to a node all the same, moving other groups' nodes along
+            unsigned seen = 0;
+            auto place = [&](auto&& self, int g) -> bool {
+                for (unsigned open; (open = has[g] & ~seen) != 0;) {
+                    const int l = __builtin_ctz(open);
+                    seen |= 1u << l;
+                    if (take[l] < 0 || self(self, take[l])) {
+                        take[l] = g;
+                        taken |= 1u << l;
+                        return true;
+                    }
+                }
+                return false;
+            };
+            place(place, g0);
+        }
+        for (int l = 0; l < n; l++)
+            if (take[l] >= 0) load[take[l]]++;
+        for (int l = 0; l < n; l++) {
+            if (r >= begin[l + 1] - begin[l]) continue;
+            if (take[l] < 0) {
+                int best = -1;
+                for (int g = 0; g < BANK_GROUPS; g++)
+                    if (left[l][g] && (best < 0 || load[g] < load[best])) best = g;
+                take[l] = best;
+                load[best]++;
+            }
+            const int g = take[l];
+            slots[begin[l] + r] = sorted[next[l][g]++];
+            if (--left[l][g] == 0) has[g] &= ~(1u << l);
+            demand[g]--;
+        }
+    }
+}
+
+}  // namespace
+
+bool in_parallel(int64_t n, int threads, const std::function<void(int64_t, int64_t)>& work) {
     const int64_t parts = std::max<int64_t>(1, std::min<int64_t>(threads, n / 4));
     std::atomic<bool> failed{false};
     auto part = [&](int64_t k) {
@@ -217,83 +293,6 @@ bool in_parallel(int64_t n, int threads, const Work& work) {
     for (auto& t : pool) t.join();
     return !failed;
 }
-
-// Order in which the eight nodes of a quarter take their corner forces, one each per round: list[l]
-// holds node l's corner slots (corner * T + tetra, bank group tetra % 8) and is put into that order.
-// Each round matches nodes to different bank groups as far as their remaining corners allow
-// (augmenting paths, the groups in most demand first); what is left over takes the least used.
-void order_corners(std::vector<uint16_t> (&list)[BANK_GROUPS], int n) {
-    int left[BANK_GROUPS][BANK_GROUPS] = {}, next[BANK_GROUPS][BANK_GROUPS], demand[BANK_GROUPS] = {};
-    size_t rounds = 0;
-    std::vector<uint16_t> sorted[BANK_GROUPS];  // each node's slots by bank group; next: the first not yet taken
-    for (int l = 0; l < n; l++) {
-        rounds = std::max(rounds, list[l].size());
-        for (uint16_t v : list[l]) left[l][v % BANK_GROUPS]++;
-        int pos = 0, fill[BANK_GROUPS];
-        for (int g = 0; g < BANK_GROUPS; g++) {
-            next[l][g] = fill[g] = pos;
-            pos += left[l][g];
-            demand[g] += left[l][g];
-        }
-        sorted[l].resize(list[l].size());
-        for (uint16_t v : list[l]) sorted[l][fill[v % BANK_GROUPS]++] = v;
-    }
-    unsigned has[BANK_GROUPS] = {};  // per group: the nodes that still have a corner in it, as bits
-    for (int l = 0; l < n; l++)
-        for (int g = 0; g < BANK_GROUPS; g++) has[g] |= (unsigned)(left[l][g] > 0) << l;
-    int order[BANK_GROUPS];
-    for (int g = 0; g < BANK_GROUPS; g++) order[g] = g;
-    for (size_t r = 0; r < rounds; r++) {
-        int take[BANK_GROUPS], load[BANK_GROUPS] = {};
-        std::fill(take, take + BANK_GROUPS, -1);
-        for (int i = 1; i < BANK_GROUPS; i++)  // nearly sorted from the round before
-            for (int k = i; k > 0 && demand[order[k]] > demand[order[k - 1]]; k--) std::swap(order[k], order[k - 1]);
-        unsigned taken = 0;
-        for (int oi = 0; oi < BANK_GROUPS && demand[order[oi]] > 0; oi++) {
-            const int g0 = order[oi];
-            const unsigned open = has[g0] & ~taken;
-            if (open) {  // a node without a group yet
-                const int l = __builtin_ctz(open);
-                take[l] = g0;
-                taken |= 1u << l;
-                continue;
-            }
-            // match the group to a node all the same, moving other groups' nodes along
-            unsigned seen = 0;
-            auto place = [&](auto&& self, int g) -> bool {
-                for (int l = 0; l < n; l++) {
-                    if (!((has[g] >> l) & 1u) || ((seen >> l) & 1u)) continue;
-                    seen |= 1u << l;
-                    if (take[l] < 0 || self(self, take[l])) {
-                        take[l] = g;
-                        taken |= 1u << l;
-                        return true;
-                    }
-                }
-                return false;
-            };
-            place(place, g0);
-        }
-        for (int l = 0; l < n; l++)
-            if (take[l] >= 0) load[take[l]]++;
-        for (int l = 0; l < n; l++) {
-            if (r >= list[l].size()) continue;
-            if (take[l] < 0) {
-                int best = -1;
-                for (int g = 0; g < BANK_GROUPS; g++)
-                    if (left[l][g] && (best < 0 || load[g] < load[best])) best = g;
-                take[l] = best;
-                load[best]++;
-            }
-            const int g = take[l];
-            list[l][r] = sorted[l][next[l][g]++];
-            if (--left[l][g] == 0) has[g] &= ~(1u << l);
-            demand[g]--;
-        }
-    }
-}
-
-}  // namespace
 
 bool build_mesh_plan(int64_t np, int64_t nt, const double* P, const uint32_t* T, int tile_tets, MeshPlan& plan,
                      std::string& err, int threads) {
@@ -388,7 +387,10 @@ bool build_mesh_plan(int64_t np, int64_t nt, const double* P, const uint32_t* T,
     auto build_tiles = [&](int64_t b0, int64_t b1) {
         std::vector<uint32_t> ids;
         ids.reserve(4 * (size_t)tile_tets);
-        std::vector<uint16_t> corner, weights;
+        // the tile's working arrays, kept from tile to tile: with allocations of their own for each, threads
+        // planning small meshes side by side waited for the allocator (eight meshes of 14k tetras 10 ms)
+        std::vector<uint16_t> corner, weights, loc_of, slots, sorted;
+        std::vector<uint32_t> cnt_by_id, by_count, node_at, begin, fill, first;
         for (int64_t b = b0; b < b1; b++) {
             const int64_t t0 = b > 0 ? tile_end[b - 1] : 0;
             const int64_t cnt = tile_end[b] - t0;
@@ -406,7 +408,7 @@ bool build_mesh_plan(int64_t np, int64_t nt, const double* P, const uint32_t* T,
             // largest count, so grouping similar counts into the same warp saves iterations. Eight at
             // a time they are permuted against bank conflicts (number_nodes).
             corner.resize(4 * (size_t)cnt);
-            std::vector<uint32_t> cnt_by_id(nn, 0);
+            cnt_by_id.assign(nn, 0);
             for (int64_t j = 0; j < cnt; j++)
                 for (int k = 0; k < 4; k++) {
                     const uint32_t g = (uint32_t)plan.node_int[T[k * nt + order[t0 + j]]];
@@ -414,19 +416,20 @@ bool build_mesh_plan(int64_t np, int64_t nt, const double* P, const uint32_t* T,
                     corner[4 * j + k] = a;
                     cnt_by_id[a]++;
                 }
-            std::vector<uint32_t> by_count(nn);
+            by_count.resize(nn);
             std::iota(by_count.begin(), by_count.end(), 0u);
-            std::stable_sort(by_count.begin(), by_count.end(),
-                             [&](uint32_t a, uint32_t c) { return cnt_by_id[a] > cnt_by_id[c]; });
-            std::vector<uint16_t> loc_of(nn);
+            std::sort(by_count.begin(), by_count.end(), [&](uint32_t a, uint32_t c) {
+                return cnt_by_id[a] != cnt_by_id[c] ? cnt_by_id[a] > cnt_by_id[c] : a < c;
+            });
+            loc_of.resize(nn);
             number_nodes((int)cnt, (int)nn, corner.data(), by_count, loc_of, weights);
-            std::vector<uint32_t> node_at(nn);  // local number -> position in ids
+            node_at.resize(nn);  // local number -> position in ids
             for (size_t a = 0; a < nn; a++) node_at[loc_of[a]] = (uint32_t)a;
-            std::vector<uint16_t> slots(4 * (size_t)cnt);  // corner slots by local node, in (tet, corner) order
-            std::vector<uint32_t> begin(nn + 1, 0);
+            slots.resize(4 * (size_t)cnt);  // corner slots by local node, in (tet, corner) order
+            begin.assign(nn + 1, 0);
             for (size_t a = 0; a < nn; a++) begin[loc_of[a] + 1] = cnt_by_id[a];
             for (size_t q = 0; q < nn; q++) begin[q + 1] += begin[q];
-            std::vector<uint32_t> fill(begin.begin(), begin.end() - 1);
+            fill.assign(begin.begin(), begin.end() - 1);
             for (int64_t j = 0; j < cnt; j++) {
                 slot_user[s0 + j] = order[t0 + j];
                 for (int k = 0; k < 4; k++) {
@@ -438,20 +441,17 @@ bool build_mesh_plan(int64_t np, int64_t nt, const double* P, const uint32_t* T,
             // Incidence list of the tile: the local nodes of a quarter side by side, eight entries per
             // round, a node's entries one round apart; a node with fewer than its quarter's most has
             // unused entries.
-            std::vector<uint32_t> first(nn);
+            first.resize(nn);
             std::vector<uint16_t> inc;
+            inc.reserve(6 * (size_t)cnt);
             for (size_t w = 0; w < nn; w += 4 * BANK_GROUPS) {
                 const int nq = (int)std::min<size_t>(4, (nn - w + BANK_GROUPS - 1) / BANK_GROUPS);
-                std::vector<uint16_t> list[4][BANK_GROUPS];
                 int rounds[4] = {};
                 for (int u = 0; u < nq; u++) {
                     const size_t q = w + u * BANK_GROUPS;
                     const int n = (int)std::min<size_t>(BANK_GROUPS, nn - q);
-                    for (int l = 0; l < n; l++) {
-                        list[u][l].assign(slots.begin() + begin[q + l], slots.begin() + begin[q + l + 1]);
-                        rounds[u] = std::max(rounds[u], (int)list[u][l].size());
-                    }
-                    order_corners(list[u], n);
+                    for (int l = 0; l < n; l++) rounds[u] = std::max(rounds[u], (int)(begin[q + l + 1] - begin[q + l]));
+                    order_corners(slots.data(), begin.data() + q, n, sorted);
                 }
                 // the quarters of a warp read their lists in step: lay them out so that as few as possible
                 // start in the same bank group
@@ -475,8 +475,10 @@ bool build_mesh_plan(int64_t np, int64_t nt, const double* P, const uint32_t* T,
                     const size_t base = inc.size();
                     inc.resize(base + (size_t)rounds[u] * BANK_GROUPS, 0);
                     for (int l = 0; l < BANK_GROUPS && w + u * BANK_GROUPS + l < nn; l++) {
-                        first[w + u * BANK_GROUPS + l] = (uint32_t)(base + l);
-                        for (size_t r = 0; r < list[u][l].size(); r++) inc[base + r * BANK_GROUPS + l] = (uint16_t)(16 * list[u][l][r]);
+                        const size_t q = w + u * BANK_GROUPS + l;
+                        first[q] = (uint32_t)(base + l);
+                        for (uint32_t i = begin[q]; i < begin[q + 1]; i++)
+                            inc[base + (i - begin[q]) * BANK_GROUPS + l] = (uint16_t)(16 * slots[i]);
                     }
                 }
             }
