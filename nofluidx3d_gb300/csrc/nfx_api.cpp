@@ -235,7 +235,10 @@ int use_runs(nfx_sim* s, bool& yes) {
     if (s->cell.si_contact >= 0 || !s->plan.all_nodes_used) return NFX_OK;
     if (s->run_tiles[0] < 0) CUDA_TRY(run_tiles_max(s->mesh, s->cell.mat.model, s->run_tiles));
     yes = s->mesh.ntiles <= std::max(s->run_tiles[0], s->run_tiles[1]);
-    if (yes && !s->d_run_acc) return dalloc(s, &s->d_run_acc, 9 * (size_t)s->plan.np, &s->mesh_allocs);
+    if (yes && !s->d_run_acc && dalloc(s, &s->d_run_acc, 9 * (size_t)s->plan.np, &s->mesh_allocs) != NFX_OK) {
+        cudaGetLastError();  // no room for the accumulators: the two passes need none
+        yes = false;
+    }
     return NFX_OK;
 }
 

@@ -18,7 +18,8 @@
 // simulation is a table of one cell, a batch many, and both run this same code. The kernel
 // boundary is the step's only global barrier. Time t comes from device memory (start of the
 // captured chunk) plus the launch's offset, so a captured CUDA graph of G steps can be replayed
-// for any chunk.
+// for any chunk. A single cell whose tiles all fit the GPU at once takes its steps in k_run instead, one
+// cooperative launch for a run of steps, with the two passes for the steps that record.
 #include <cuda_runtime.h>
 
 #include "nfx_internal.h"
