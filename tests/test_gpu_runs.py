@@ -58,3 +58,32 @@ def test_run_equals_two_passes(options, extra):
         assert out[0][0] == 0 and np.isfinite(out[0][1]).all()
     elif extra != "table":
         assert np.abs(out[0][7]).max() > 0 and len(out[0][7]) == 3
+
+
+@pytest.mark.parametrize("radius", [5.0, 13.0])
+def test_handles_side_by_side(radius):
+    """Cells stepped by several threads at once, where some calls meet other handles at work and take the
+    two passes, against the same cell stepped alone."""
+    import threading
+    w = Workload("run", radius=radius, material="mr_vp", indenter="sphere", sphere_radius=4.0, speed=2e-3)
+    mesh = w.mesh()
+    sims = [CellSim(0) for _ in range(4)]
+    for s in sims:
+        w.configure(s, mesh, max_rows=50)
+
+    def steps(s):
+        for n in (50, 4, 1, 145):
+            s.step(n)
+
+    steps(sims[0])
+    want = state(sims[0])
+    threads = [threading.Thread(target=steps, args=(s,)) for s in sims[1:]]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for s in sims[1:]:
+        for a, b in zip(state(s), want):
+            assert np.array_equal(a, b)
+    for s in sims:
+        s.close()
