@@ -1302,12 +1302,15 @@ __global__ void k_plastic_from_user(int ns, long long nt, StateDev s, const int*
 // Launchers
 // ------------------------------------------------------------------------------------------
 // Dynamic shared memory of a tile's incidence list: 10 bytes a tetra on the meshes measured, at most
-// 24 (a node in every tetra of its tile), which only with 512-tetra tiles can pass 48 KB a CTA.
+// 24 (a node in every tetra of its tile), which only with 512-tetra tiles can pass 48 KB a CTA. The limit
+// belongs to the kernel and is shared by all handles and threads, so it is set to that bound, not
+// to the mesh's own need.
+constexpr int INC_BYTES_PER_TET = 24;
 static size_t inc_bytes(const MeshDev& m) { return (size_t)m.inc_stride * sizeof(unsigned short); }
 template <int TILE>
-static cudaError_t allow_inc(const void* kernel, const MeshDev& m) {
+static cudaError_t allow_inc(const void* kernel) {
     if (TILE < 512) return cudaSuccess;
-    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)inc_bytes(m));
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, INC_BYTES_PER_TET * TILE);
 }
 
 template <int MODEL, int TILE>
@@ -1317,7 +1320,7 @@ static cudaError_t launch_tet(const MeshDev& m, const StateDev& s, const BatchDe
     cfg.gridDim = dim3((unsigned)m.ntiles);
     cfg.blockDim = dim3(TILE);
     cfg.dynamicSmemBytes = inc_bytes(m);
-    cudaError_t e = allow_inc<TILE>((const void*)k_tet_pass<MODEL, TILE>, m);
+    cudaError_t e = allow_inc<TILE>((const void*)k_tet_pass<MODEL, TILE>);
     if (e != cudaSuccess) return e;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
@@ -1355,7 +1358,7 @@ cudaError_t launch_tet_pass(const MeshDev& m, const StateDev& s, const BatchDev&
 template <int TILE>
 static cudaError_t launch_si(const MeshDev& m, const StateDev& s, const BatchDev& b, int t_offset, int mode, int contact,
                              cudaStream_t st, bool pdl) {
-    const cudaError_t e = allow_inc<TILE>((const void*)k_si_pass<TILE>, m);
+    const cudaError_t e = allow_inc<TILE>((const void*)k_si_pass<TILE>);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)m.ntiles);
