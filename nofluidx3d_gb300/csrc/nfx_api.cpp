@@ -713,13 +713,26 @@ int nfx_set_viscoplastic(nfx_sim* s, const double* par) {
     if ((rc = set_device(s)) != NFX_OK) return rc;
     const size_t ntp = (size_t)s->plan.nslots + ARRAY_PAD;
     if (!s->st.vp_a) {
-        if ((rc = dalloc(s, &s->st.vp_a, ntp, &s->mesh_allocs)) || (rc = dalloc(s, &s->st.vp_b, ntp, &s->mesh_allocs)) ||
-            (rc = dalloc(s, &s->st.vp_c, ntp, &s->mesh_allocs)) || (rc = dalloc(s, &s->st.fields, ntp, &s->mesh_allocs)) ||
-            (rc = dalloc(s, &s->d_tet_user, (size_t)s->plan.nslots, &s->mesh_allocs)))
-            return rc;
+        // all of the state or none of it: nothing is put in place before every array is there
         const std::vector<int> tu(s->plan.tet_user.begin(), s->plan.tet_user.end());
-        CUDA_TRY(cudaMemcpyAsync(s->d_tet_user, tu.data(), tu.size() * sizeof(int), cudaMemcpyHostToDevice, s->stream));
-        CUDA_TRY(cudaStreamSynchronize(s->stream));  // tu goes out of scope
+        float4 *pa, *pb; float2 *pc, *fields; int* tet_user;
+        std::vector<void*> got;
+        auto give_back = [&](int code) {
+            for (void* p : got) cudaFree(p);
+            return code;
+        };
+        if ((rc = dalloc(s, &pa, ntp, &got)) || (rc = dalloc(s, &pb, ntp, &got)) || (rc = dalloc(s, &pc, ntp, &got)) ||
+            (rc = dalloc(s, &fields, ntp, &got)) || (rc = dalloc(s, &tet_user, tu.size(), &got)))
+            return give_back(rc);
+        cudaError_t e = cudaMemcpyAsync(tet_user, tu.data(), tu.size() * sizeof(int), cudaMemcpyHostToDevice, s->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);  // tu goes out of scope
+        if (e != cudaSuccess) return give_back(fail(NFX_ERR_CUDA, std::string("viscoplastic state: ") + cudaGetErrorString(e)));
+        s->mesh_allocs.insert(s->mesh_allocs.end(), got.begin(), got.end());
+        s->st.vp_a = pa;
+        s->st.vp_b = pb;
+        s->st.vp_c = pc;
+        s->st.fields = fields;
+        s->d_tet_user = tet_user;
     }
     CUDA_TRY(cudaMemsetAsync(s->st.vp_a, 0, ntp * sizeof(float4), s->stream));
     CUDA_TRY(cudaMemsetAsync(s->st.vp_b, 0, ntp * sizeof(float4), s->stream));
