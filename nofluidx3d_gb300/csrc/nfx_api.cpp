@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -87,7 +88,10 @@ struct nfx_sim {
     unsigned* d_arrivals = nullptr;
     unsigned arrivals = 0;
     int run_tiles[2] = {-1, -1};
-    unsigned long long* d_run_acc = nullptr;  // three accumulators, allocated with the first run of a mesh
+    unsigned long long* d_run_acc = nullptr;  // three accumulators, allocated with a mesh that may take runs
+    // Calls that enqueued steps, counted after their launches, and the count up to which the stream was
+    // last found idle by another handle (others_busy).
+    std::atomic<unsigned long long> work{0}, idle{0};
     // Page-locked host memory that kernels write small results into: the readout (first word) and,
     // of small meshes, the positions. The result is there when the stream has been waited for, without
     // a copy behind the kernel.
@@ -216,6 +220,7 @@ int enqueue_steps(nfx_sim* s, int n) {
         CUDA_TRY(launch_nodes(s, k, NODE_UPDATE, -1, true));
     }
     CUDA_TRY(launch_advance_time(s->st, n, s->fields_every, s->record_every, s->stream));
+    s->work++;
     return NFX_OK;
 }
 
@@ -249,36 +254,36 @@ struct RelaxedCapture {
     ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
 };
 
-// Whether another handle has work on the same device (at most 32 are asked).
+// Whether another handle has work on the same device. A stream found idle is asked again only after its
+// handle has enqueued more (an ask takes 1.3 us: 40 idle handles made a one-step call of 22 us 75);
+// at most 32 are asked.
 bool others_busy(const nfx_sim* s) {
     RelaxedCapture relaxed;
     std::lock_guard<std::mutex> hold(handles().lock);
     int asked = 0;
-    for (const nfx_sim* o : handles().all) {
+    for (nfx_sim* o : handles().all) {
         if (o == s || o->device != s->device) continue;
+        const unsigned long long work = o->work.load();
+        if (work == o->idle.load()) continue;
         if (cudaStreamQuery(o->stream) == cudaErrorNotReady) {
             cudaGetLastError();
             return true;
         }
+        o->idle.store(work);
         if (++asked == 32) break;
     }
     return false;
 }
 
-// Whether the cell's steps go in cooperative runs (k_run): all its tiles must fit the GPU at once.
-int use_runs(nfx_sim* s, bool& yes) {
+// Whether nsteps steps of the cell go in cooperative runs (k_run): all its tiles must fit the GPU at once.
+int use_runs(nfx_sim* s, int64_t nsteps, bool& yes) {
     yes = false;
-    if (s->cell.si_contact >= 0 || !s->plan.all_nodes_used) return NFX_OK;
+    if (nsteps < RUN_STEPS_MIN || s->cell.si_contact >= 0 || !s->d_run_acc) return NFX_OK;
     if (s->run_tiles[0] < 0) CUDA_TRY(run_tiles_max(s->mesh, s->cell.mat.model, s->run_tiles));
     yes = s->mesh.ntiles <= std::max(s->run_tiles[0], s->run_tiles[1]);
     // Runs of cells of which fewer than four fit the GPU side by side take turns, while the two passes of
     // several handles overlap: four R = 14 cells stepped by four threads 53 ms in runs, 32 in passes.
     if (yes && 4 * s->mesh.ntiles > s->run_tiles[0] && others_busy(s)) yes = false;
-    RelaxedCapture relaxed;
-    if (yes && !s->d_run_acc && dalloc(s, &s->d_run_acc, 9 * (size_t)s->plan.np, &s->mesh_allocs) != NFX_OK) {
-        cudaGetLastError();  // no room for the accumulators: the two passes need none
-        yes = false;
-    }
     return NFX_OK;
 }
 
@@ -305,6 +310,7 @@ int run_steps(nfx_sim* s, int64_t n) {
                                 (int)plain, s->stream));
             s->arrivals += (unsigned)plain * (unsigned)s->mesh.ntiles;
             CUDA_TRY(launch_advance_time(s->st, plain, s->fields_every, s->record_every, s->stream));
+            s->work++;
             done += plain;
         } else {
             // up to the next stretch worth a run: the due steps and the few between them
@@ -677,6 +683,10 @@ int nfx_set_mesh(nfx_sim* s, int64_t np, int64_t nt, const double* points, const
     s->cell.tile_end = (int)P.ntiles;
     s->cell_dirty = true;
     s->have_mesh = true;
+    // The accumulators of runs of steps, here rather than in the first step, so that stepping allocates
+    // nothing; without room for them the cell keeps the two passes, which need none.
+    if (P.all_nodes_used && P.ntiles <= run_tiles_bound(s->mesh) && dalloc(s, &s->d_run_acc, 9 * (size_t)np, &A) != NFX_OK)
+        cudaGetLastError();
     // the viscoplastic state follows the mesh
     if (s->have_material && s->cell.mat.model == MODEL_VP) {
         s->have_material = false;
@@ -898,7 +908,7 @@ int nfx_step(nfx_sim* s, int64_t nsteps) {
     const long long t_begin = s->time;
     int64_t left = nsteps;
     bool runs = false;
-    if ((rc = use_runs(s, runs)) != NFX_OK) return rc;
+    if ((rc = use_runs(s, nsteps, runs)) != NFX_OK) return rc;
     if (runs) {
         if ((rc = run_steps(s, nsteps)) != NFX_OK) return rc;
         left = 0;
@@ -906,6 +916,7 @@ int nfx_step(nfx_sim* s, int64_t nsteps) {
     while (left >= GRAPH_STEPS) {
         if (!s->graph_valid && (rc = build_graph(s)) != NFX_OK) return rc;
         CUDA_TRY(cudaGraphLaunch(s->graph, s->stream));
+        s->work++;
         left -= GRAPH_STEPS;
     }
     if (left > 0 && (rc = enqueue_steps(s, (int)left)) != NFX_OK) return rc;

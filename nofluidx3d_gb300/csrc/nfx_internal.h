@@ -244,7 +244,9 @@ cudaError_t launch_advance_time(const StateDev& s, long long n, long long fields
 // barrier's arrival counter, base its value at the launch; the launch adds nsteps * ntiles. acc: three
 // accumulators of 3 * np words, all zero at the launch. A barrier that is not met within about a
 // second raises STATUS_TIMEOUT and ends the run.
+// run_tiles_bound: at least as many as run_tiles_max for any model, without loading a kernel.
 cudaError_t run_tiles_max(const MeshDev& m, int model, int (&tiles)[2]);
+int run_tiles_bound(const MeshDev& m);
 cudaError_t launch_run(const MeshDev& m, const StateDev& s, const BatchDev& b, int model, int form, unsigned* count,
                        unsigned base, unsigned long long* acc, int nsteps, cudaStream_t stream);
 // Integrated sphere contact over all tiles (tiles of cells without one return at once). Inside a

@@ -1387,9 +1387,20 @@ static cudaError_t run_capacity(const MeshDev& m, int (&tiles)[2]) {
     return e;
 }
 
+static bool run_mesh(const MeshDev& m) {
+    return m.tile_tets == RUN_TILE && (m.np + 31) / 32 <= (RUN_TILE / 32) * m.ntiles;
+}
+int run_tiles_bound(const MeshDev& m) {
+    int dev = 0, sms = 0;
+    if (!run_mesh(m) || cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return 0;
+    return sms * RUN_PER_SM[1];
+}
+
 cudaError_t run_tiles_max(const MeshDev& m, int model, int (&tiles)[2]) {
     tiles[0] = tiles[1] = 0;
-    if (m.tile_tets != RUN_TILE || (m.np + 31) / 32 > (RUN_TILE / 32) * m.ntiles) return cudaSuccess;
+    if (!run_mesh(m)) return cudaSuccess;
     switch (model) {
         case MODEL_MR: return run_capacity<MODEL_MR>(m, tiles);
         case MODEL_SVK: return run_capacity<MODEL_SVK>(m, tiles);

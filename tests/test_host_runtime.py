@@ -70,3 +70,68 @@ def test_failed_allocation_of_the_viscoplastic_state(fake, nth):
         s.tet_field(k)
     s.set_plastic_tensor_soa(s.plastic_tensor_soa())
     s.close()
+
+
+def test_steps_allocate_nothing(fake):
+    """Every array of the steps is there once the cell is set up, whichever way its steps go; a call for
+    fewer steps than a run takes asks no other handle's stream."""
+    fake.fake_run_tiles(4, 912)
+    others = [cell() for _ in range(3)]
+    s = cell()
+    fake.fake_reset()
+    s.step(1)
+    for o in others:
+        o.step(3)
+    assert fake.fake_count(QUERIES) == 0 and fake.fake_count(TETS) == 10
+    for n in (10, 500):
+        s.step(n)
+    assert fake.fake_count(RUNS) > 0 and fake.fake_count(MALLOCS) == 0
+    for o in others + [s]:
+        o.close()
+
+
+def test_no_room_for_the_accumulators_of_runs(fake):
+    """The mesh is set and the two passes serve."""
+    fake.fake_run_tiles(608, 912)
+    s = core.CellSim(0)
+    w = Workload("host", radius=3.0, material="nh")
+    m = w.mesh()
+    s.set_mesh(m.points, m.tets)
+    n = fake.fake_count(MALLOCS)
+    fake.fake_reset()
+    s.set_mesh(m.points, m.tets)
+    arrays = fake.fake_count(MALLOCS)
+    assert n > arrays
+    fake.fake_fail_malloc(arrays - 1)  # the last one
+    w.configure(s, m, max_rows=10)
+    fake.fake_reset()
+    s.step(20)
+    assert fake.fake_count(RUNS) == 0 and fake.fake_count(TETS) == 20
+    s.close()
+
+
+def test_idle_handles_are_asked_once(fake):
+    """A cell of which fewer than four fit the GPU side by side asks whether others are at work: a handle
+    found idle is asked again only when it has stepped since."""
+    fake.fake_run_tiles(4, 912)
+    others = [cell() for _ in range(5)]
+    s = cell()
+    for o in others:
+        o.step(2)
+    fake.fake_reset()
+    for _ in range(20):
+        s.step(10)
+    assert fake.fake_count(QUERIES) == 5 and fake.fake_count(RUNS) == 20
+    others[2].step(2)
+    fake.fake_busy(1)
+    fake.fake_reset()
+    s.step(10)
+    assert fake.fake_count(QUERIES) == 1 and fake.fake_count(RUNS) == 0
+    s.step(10)
+    assert fake.fake_count(QUERIES) == 2  # still at work, so asked again
+    fake.fake_busy(0)
+    s.step(10)
+    s.step(10)
+    assert fake.fake_count(QUERIES) == 3 and fake.fake_count(RUNS) == 2
+    for o in others + [s]:
+        o.close()
