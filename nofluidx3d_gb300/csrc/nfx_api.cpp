@@ -10,6 +10,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <limits>
 #include <mutex>
 #include <string>
 #include <thread>
@@ -275,12 +276,31 @@ bool others_busy(const nfx_sim* s) {
     return false;
 }
 
+// The most steps in a row that neither record a row nor write fields (both have the same interval).
+long long longest_stretch(const nfx_sim* s) {
+    const bool rows = s->cell.record_contact >= 0 && s->record_every > 0;
+    const bool fields = s->cell.mat.model == MODEL_VP && s->fields_every > 0;
+    if (!rows && !fields) return std::numeric_limits<long long>::max();
+    return (rows ? s->record_every : s->fields_every) - (rows ? 1 : 0) - (fields ? 1 : 0);
+}
+
+// The shortest such stretch for which a cell that records on and on takes runs: a run, and the launches
+// of the due steps beside it, cost about 17 us that the steps of the run have to win back from the
+// graph's two passes. Measured, us a step, graph / runs, by the steps of a stretch: 14 tiles elastic
+// 6.71 / 6.77 at 6, 6.64 / 6.48 at 7, 6.61 / 6.17 at 8; 102 elastic 6.49 / 6.94 at 7, 6.44 / 6.52 at 8, 6.41 /
+// 6.27 at 9; 102 viscoplastic 7.82 / 8.23 at 7, 7.78 / 7.75 at 8, 7.74 / 7.66 at 9; 338 viscoplastic 9.54 / 9.97 at 5,
+// 9.47 / 9.52 at 6, 9.42 / 9.15 at 7; 541 elastic 9.77 / 9.95 at 5, 9.62 / 9.25 at 6; 809 viscoplastic
+// 12.08 / 12.54 at 5, 12.00 / 12.03 at 6, 11.93 / 11.55 at 7.
+long long stretch_min(const nfx_sim* s) {
+    return 4 * s->mesh.ntiles > s->run_tiles[0] ? 6 : 9;  // more than one tile per SM or not
+}
+
 // Whether nsteps steps of the cell go in cooperative runs (k_run): all its tiles must fit the GPU at once.
 int use_runs(nfx_sim* s, int64_t nsteps, bool& yes) {
     yes = false;
     if (nsteps < RUN_STEPS_MIN || s->cell.si_contact >= 0 || !s->d_run_acc) return NFX_OK;
     if (s->run_tiles[0] < 0) CUDA_TRY(run_tiles_max(s->mesh, s->cell.mat.model, s->run_tiles));
-    yes = s->mesh.ntiles <= std::max(s->run_tiles[0], s->run_tiles[1]);
+    yes = s->mesh.ntiles <= std::max(s->run_tiles[0], s->run_tiles[1]) && longest_stretch(s) >= stretch_min(s);
     // Runs of cells of which fewer than four fit the GPU side by side take turns, while the two passes of
     // several handles overlap: four R = 14 cells stepped by four threads 53 ms in runs, 32 in passes.
     if (yes && 4 * s->mesh.ntiles > s->run_tiles[0] && others_busy(s)) yes = false;

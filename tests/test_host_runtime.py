@@ -135,3 +135,23 @@ def test_idle_handles_are_asked_once(fake):
     assert fake.fake_count(QUERIES) == 3 and fake.fake_count(RUNS) == 2
     for o in others + [s]:
         o.close()
+
+
+@pytest.mark.parametrize("material,tiles,every,runs", [
+    ("nh", 608, 1, False), ("nh", 608, 5, False), ("nh", 608, 9, False), ("nh", 608, 10, True), ("mr_vp", 608, 10, False),
+    ("mr_vp", 608, 11, True), ("nh", 4, 6, False), ("nh", 4, 7, True), ("mr_vp", 4, 7, False), ("mr_vp", 4, 8, True)])
+def test_short_record_intervals_keep_the_graph(fake, material, tiles, every, runs):
+    """Where the steps between two that record are too few for a run to pay, a call replays the graph of
+    the two passes, whose remainder is launched step by step."""
+    fake.fake_run_tiles(tiles, 912)
+    s = cell(material=material, record_every=every)
+    fake.fake_reset()
+    s.step(430)
+    steps = fake.fake_count(TETS) + 100 * fake.fake_count(GRAPHS) + fake.fake_count(RUN_STEPS)
+    assert steps == 430 and fake.fake_count(TETS) == fake.fake_count(NODES)
+    if runs:
+        assert fake.fake_count(GRAPHS) == 0 and fake.fake_count(RUNS) == len(range(0, 430 - 4, every))
+    else:
+        assert fake.fake_count(RUNS) == 0 and fake.fake_count(GRAPHS) == 4 and fake.fake_count(TETS) == 30
+        assert fake.fake_count(ADVANCES) == 1
+    s.close()
