@@ -238,6 +238,13 @@ int nfx_profile_tet_pass(nfx_sim* sim, int launches, float* ms);
  * with no counterpart in the reference. */
 int nfx_divide_check(int device, int64_t n, const float* a, const float* b, float* q);
 
+/* Enqueues a run of four steps in one launch (see nfx_step) whose wait for its CTAs is never met and gives
+ * up after `polls` (1..65536) polls, and counts four steps as taken: the handle is left as by a wait
+ * that ran out, with NFX_STATUS_TIMEOUT set, an invalid state, and runs that return at once until
+ * nfx_set_mesh or nfx_checkpoint_load. NFX_ERR_STATE when the cell's steps do not go in runs. A
+ * self-check with no counterpart in the reference. */
+int nfx_run_timeout_check(nfx_sim* sim, int polls);
+
 /* Number of mesh tiles and distinct-node entries (diagnostics for the tile layout). */
 int nfx_mesh_info(nfx_sim* sim, int64_t* ntiles, int64_t* tile_nodes);
 

@@ -18,7 +18,7 @@ ERR_NAMES = {1: "NFX_ERR_ARG", 2: "NFX_ERR_CUDA", 3: "NFX_ERR_STATE", 4: "NFX_ER
 
 MODEL_MR, MODEL_SVK, MODEL_SVKK, MODEL_VP = 0, 1, 2, 3
 CONTACT_SUBSTRATE, CONTACT_PLANE, CONTACT_SPHERE, CONTACT_SPHERE_INTEGRAL = 0, 1, 2, 3
-STATUS_NONFINITE, STATUS_INVERTED, STATUS_CURVE_FULL = 1, 2, 4
+STATUS_NONFINITE, STATUS_INVERTED, STATUS_CURVE_FULL, STATUS_TIMEOUT = 1, 2, 4, 8
 FIELD_VON_MISES, FIELD_PRESSURE, FIELD_PLASTIC_STRAIN = 0, 1, 2
 
 
@@ -77,6 +77,7 @@ _SIGS = {
     "nfx_snapshot_wait": ([_vp], C.c_int),
     "nfx_host_alloc": ([C.c_size_t, C.POINTER(_vp)], C.c_int),
     "nfx_host_free": ([_vp], C.c_int),
+    "nfx_run_timeout_check": ([_vp, C.c_int], C.c_int),
     "nfx_divide_check": ([C.c_int, _i64, _vp, _vp, _vp], C.c_int),
     "nfx_indenter_force_noalloc": ([C.c_int, _i64, _vp, C.c_int, C.c_double, C.c_double, C.c_double, _vp, _vp],
                                    C.c_int),

@@ -1278,6 +1278,26 @@ int nfx_profile_tet_pass(nfx_sim* s, int launches, float* ms) {
     return NFX_OK;
 }
 
+int nfx_run_timeout_check(nfx_sim* s, int polls) {
+    int rc;
+    if ((rc = require_ready(s)) != NFX_OK) return rc;
+    CHECK_ARG(polls >= 1 && polls <= (1 << 16), "polls out of range [1, 65536]");
+    if ((rc = set_device(s)) != NFX_OK) return rc;
+    if ((rc = upload_cell(s)) != NFX_OK) return rc;
+    bool runs = false;
+    if ((rc = use_runs(s, RUN_STEPS_MIN, runs)) != NFX_OK) return rc;
+    if (!runs) return fail(NFX_ERR_STATE, "the cell's steps do not go in runs");
+    CUDA_TRY(cudaMemsetAsync(s->d_run_acc, 0, 9 * (size_t)s->plan.np * sizeof(unsigned long long), s->stream));
+    // one arrival more than there are CTAs: the first barrier is never met
+    CUDA_TRY(launch_run(s->mesh, s->st, table_view(s), s->cell.mat.model, s->mesh.ntiles <= s->run_tiles[0] ? 0 : 1,
+                        s->d_arrivals, s->arrivals + 1, s->d_run_acc, RUN_STEPS_MIN, s->stream, (unsigned)polls));
+    s->arrivals += (unsigned)RUN_STEPS_MIN * (unsigned)s->mesh.ntiles;
+    CUDA_TRY(launch_advance_time(s->st, RUN_STEPS_MIN, s->fields_every, s->record_every, s->stream));
+    s->work++;
+    s->time += RUN_STEPS_MIN;
+    return NFX_OK;
+}
+
 int nfx_divide_check(int device, int64_t n, const float* a, const float* b, float* q) {
     CHECK_ARG(a && b && q, "null argument");
     CHECK_ARG(n >= 0 && n <= (int64_t)1 << 26, "n out of range [0, 2^26]");

@@ -242,13 +242,15 @@ cudaError_t launch_advance_time(const StateDev& s, long long n, long long fields
 // tiles a mesh like m may have for the launch's two forms (0: not this mesh), and nsteps steps from
 // the clock's time in form 0 or 1, none of which may record a row or write fields. count: the grid
 // barrier's arrival counter, base its value at the launch; the launch adds nsteps * ntiles. acc: three
-// accumulators of 3 * np words, all zero at the launch. A barrier that is not met within about a
-// second raises STATUS_TIMEOUT and ends the run.
+// accumulators of 3 * np words, all zero at the launch. A barrier that is not met within `polls` polls
+// raises STATUS_TIMEOUT and ends the run; a run that finds that status set returns at once.
 // run_tiles_bound: at least as many as run_tiles_max for any model, without loading a kernel.
+constexpr unsigned RUN_POLLS = 1u << 21;  // about a second
 cudaError_t run_tiles_max(const MeshDev& m, int model, int (&tiles)[2]);
 int run_tiles_bound(const MeshDev& m);
 cudaError_t launch_run(const MeshDev& m, const StateDev& s, const BatchDev& b, int model, int form, unsigned* count,
-                       unsigned base, unsigned long long* acc, int nsteps, cudaStream_t stream);
+                       unsigned base, unsigned long long* acc, int nsteps, cudaStream_t stream,
+                       unsigned polls = RUN_POLLS);
 // Integrated sphere contact over all tiles (tiles of cells without one return at once). Inside a
 // step (readout false): its forces join the accumulator and, on record steps, the tile partials
 // of the readout are written. readout true: only the tile partials of contact index `contact` at

@@ -1031,12 +1031,11 @@ constexpr int RUN_TILE = DEFAULT_TILE_TETS;
 // viscoplastic 11.7 / - / 8.4; under a flat indenter R = 8 5.9 / 4.2. What is left of the 4.2 is the
 // barrier (1.3), the sums' reads (1.2 with the contacts), the force sums (0.6) and the law (0.3).
 constexpr int RUN_PER_SM[2] = {4, 6};
-// Polls after which a barrier gives up (about a second), raises STATUS_TIMEOUT and ends the run.
-constexpr unsigned RUN_SPIN_LIMIT = 1u << 21;
 
 // Waits until every CTA of the launch has arrived (target: the arrival count that makes it so). What a
-// thread wrote before is visible to all after. False when the wait ran out; uniform over the CTA.
-__device__ __forceinline__ bool grid_barrier(unsigned* count, unsigned target, int* s_ok) {
+// thread wrote before is visible to all after. False when the wait ran out, after `most` polls; uniform
+// over the CTA.
+__device__ __forceinline__ bool grid_barrier(unsigned* count, unsigned target, unsigned most, int* s_ok) {
     __syncthreads();
     if (threadIdx.x == 0) {
         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
@@ -1045,7 +1044,7 @@ __device__ __forceinline__ bool grid_barrier(unsigned* count, unsigned target, i
         do {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
             ok = (int)(v - target) >= 0;
-        } while (!ok && ++polls < RUN_SPIN_LIMIT);
+        } while (!ok && ++polls < most);
         *s_ok = ok;
     }
     __syncthreads();
@@ -1054,7 +1053,7 @@ __device__ __forceinline__ bool grid_barrier(unsigned* count, unsigned target, i
 
 template <int MODEL, int PER_SM>
 __global__ void __launch_bounds__(RUN_TILE, PER_SM) k_run(MeshDev m, StateDev s, BatchDev bd, unsigned* count, unsigned base,
-                                                     unsigned long long* acc, int nsteps) {
+                                                     unsigned long long* acc, int nsteps, unsigned polls) {
     __shared__ float4 s_v[RUN_TILE];
     __shared__ float4 s_cf[4 * RUN_TILE];
     __shared__ float4 s_ref[2];  // displacement of the tile's first node, hi and lo
@@ -1067,7 +1066,11 @@ __global__ void __launch_bounds__(RUN_TILE, PER_SM) k_run(MeshDev m, StateDev s,
     static_assert(sizeof(CellDev) % 4 == 0, "copied by words");
     for (int w = j; w < (int)(sizeof(CellDev) / 4); w += RUN_TILE)
         reinterpret_cast<unsigned*>(&C)[w] = reinterpret_cast<const unsigned*>(bd.cells)[w];
+    if (j == 0) s_ok = (*reinterpret_cast<volatile unsigned*>(s.status) & STATUS_TIMEOUT) == 0u;
     __syncthreads();
+    // After a wait that ran out the state is invalid and the arrivals are not what the host counts on:
+    // without this every run until the mesh is set or a checkpoint loaded would wait its time out too.
+    if (!s_ok) return;
     if (j < C.n_contacts) {
         s_meta[j][0] = C.c[j].meta[0];
         s_meta[j][1] = C.c[j].meta[1];
@@ -1148,7 +1151,7 @@ __global__ void __launch_bounds__(RUN_TILE, PER_SM) k_run(MeshDev m, StateDev s,
             s_wall[c0] = WallStep{w, (float)w, (float)C.c[c0].radius};
         }
         target += gridDim.x;
-        if (!grid_barrier(count, target, &s_ok)) break;
+        if (!grid_barrier(count, target, polls, &s_ok)) break;
         // node pass
         if (j < nn) {
             const unsigned long long* fa = sums.facc + i;
@@ -1412,7 +1415,7 @@ cudaError_t run_tiles_max(const MeshDev& m, int model, int (&tiles)[2]) {
 
 template <int MODEL>
 static cudaError_t launch_run_model(const MeshDev& m, const StateDev& s, const BatchDev& b, int form, unsigned* count,
-                                    unsigned base, unsigned long long* acc, int nsteps, cudaStream_t st) {
+                                    unsigned base, unsigned long long* acc, int nsteps, cudaStream_t st, unsigned polls) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)m.ntiles);
     cfg.blockDim = dim3(RUN_TILE);
@@ -1423,17 +1426,17 @@ static cudaError_t launch_run_model(const MeshDev& m, const StateDev& s, const B
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return form == 0 ? cudaLaunchKernelEx(&cfg, k_run<MODEL, RUN_PER_SM[0]>, m, s, b, count, base, acc, nsteps)
-                     : cudaLaunchKernelEx(&cfg, k_run<MODEL, RUN_PER_SM[1]>, m, s, b, count, base, acc, nsteps);
+    return form == 0 ? cudaLaunchKernelEx(&cfg, k_run<MODEL, RUN_PER_SM[0]>, m, s, b, count, base, acc, nsteps, polls)
+                     : cudaLaunchKernelEx(&cfg, k_run<MODEL, RUN_PER_SM[1]>, m, s, b, count, base, acc, nsteps, polls);
 }
 
 cudaError_t launch_run(const MeshDev& m, const StateDev& s, const BatchDev& b, int model, int form, unsigned* count,
-                       unsigned base, unsigned long long* acc, int nsteps, cudaStream_t st) {
+                       unsigned base, unsigned long long* acc, int nsteps, cudaStream_t st, unsigned polls) {
     switch (model) {
-        case MODEL_MR: return launch_run_model<MODEL_MR>(m, s, b, form, count, base, acc, nsteps, st);
-        case MODEL_SVK: return launch_run_model<MODEL_SVK>(m, s, b, form, count, base, acc, nsteps, st);
-        case MODEL_SVKK: return launch_run_model<MODEL_SVKK>(m, s, b, form, count, base, acc, nsteps, st);
-        case MODEL_VP: return launch_run_model<MODEL_VP>(m, s, b, form, count, base, acc, nsteps, st);
+        case MODEL_MR: return launch_run_model<MODEL_MR>(m, s, b, form, count, base, acc, nsteps, st, polls);
+        case MODEL_SVK: return launch_run_model<MODEL_SVK>(m, s, b, form, count, base, acc, nsteps, st, polls);
+        case MODEL_SVKK: return launch_run_model<MODEL_SVKK>(m, s, b, form, count, base, acc, nsteps, st, polls);
+        case MODEL_VP: return launch_run_model<MODEL_VP>(m, s, b, form, count, base, acc, nsteps, st, polls);
         default: return cudaErrorInvalidValue;
     }
 }

@@ -99,7 +99,7 @@ cudaError_t run_tiles_max(const MeshDev&, int, int (&tiles)[2]) {
 }
 int run_tiles_bound(const MeshDev&) { return run_tiles[1]; }
 cudaError_t launch_run(const MeshDev& m, const StateDev& s, const BatchDev& b, int, int, unsigned* count, unsigned,
-                       unsigned long long* acc, int nsteps, cudaStream_t) {
+                       unsigned long long* acc, int nsteps, cudaStream_t, unsigned) {
     counts[RUN_STEPS] += nsteps;
     return launched(RUNS, m.lconn && s.ua && b.cells && count && acc);
 }
