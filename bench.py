@@ -92,17 +92,6 @@ def load_traffic(workload_key: str) -> float | None:
     return profile_figure(workload_key, "dram_bytes_per_tetra")
 
 
-def step_launches(sim, steps: int, record_every: int, integrated: bool, device: int) -> int:
-    """Launches of `steps` steps: the two passes, and the clock once per graph of 100 steps. A cell whose
-    tiles all fit the GPU at once (six per SM) takes one launch and one of the clock for the steps
-    between two that record, and the two passes and the clock for each that does."""
-    import torch
-    if integrated or sim.mesh_info()[0] > 6 * torch.cuda.get_device_properties(device).multi_processor_count:
-        return 2 * steps + (steps + 99) // 100
-    whole, rest = divmod(steps, record_every)
-    return 5 * whole + (5 if rest > 1 else 3 if rest else 0)
-
-
 def fp32_rate(flops_per_tet: float | None, nt: int, tet_ms: float, device: int, clk: dict) -> dict | None:
     """Achieved FP32 rate of the element pass: ncu-counted FP32 FLOPs per tetra (2 per FFMA, 1 per
     FADD/FMUL) x tetra / its average launch time, against the nominal FMA peak of the device
@@ -492,6 +481,7 @@ def main():
     after = args.steps + args.profile_steps + args.e2e_steps + 400
     while window_ms < 1e3 * args.clock_window_s and sim.time + 1000 + after <= w.steps:
         window_ms += sim.time_steps(1000)
+    launches = sim.step_counts()["launches"]
     barrier(dist, local)
     ms = sim.time_steps(args.steps)
     barrier(dist, local)
@@ -500,7 +490,7 @@ def main():
         clk["window"] = f"{window_ms / 1e3:.1f} s of the same steps just before the timed region, and the timed region"
     ms = reduce_max(dist, ms, local)
     value = world * nt * args.steps / (ms / 1e3)
-    launches = step_launches(sim, args.steps, w.record_every, w.indenter == "sphere_integral", local)
+    launches = sim.step_counts()["launches"] - launches
 
     # per-kernel CUDA-event profile of the element and node passes, then the element pass alone
     # over back-to-back launches (its effects undone)

@@ -245,6 +245,11 @@ int nfx_divide_check(int device, int64_t n, const float* a, const float* b, floa
  * self-check with no counterpart in the reference. */
 int nfx_run_timeout_check(nfx_sim* sim, int polls);
 
+/* What the steps of the handle's nfx_step and nfx_time_steps calls were made of since it was created:
+ * counts[0] kernel launches, counts[1] and counts[2] steps taken in runs of one launch with up to four and
+ * up to six tiles per SM, counts[3] steps taken by the element and node passes. */
+int nfx_step_counts(nfx_sim* sim, int64_t counts[4]);
+
 /* Number of mesh tiles and distinct-node entries (diagnostics for the tile layout). */
 int nfx_mesh_info(nfx_sim* sim, int64_t* ntiles, int64_t* tile_nodes);
 

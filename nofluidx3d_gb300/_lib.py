@@ -77,6 +77,7 @@ _SIGS = {
     "nfx_snapshot_wait": ([_vp], C.c_int),
     "nfx_host_alloc": ([C.c_size_t, C.POINTER(_vp)], C.c_int),
     "nfx_host_free": ([_vp], C.c_int),
+    "nfx_step_counts": ([_vp, C.POINTER(_i64)], C.c_int),
     "nfx_run_timeout_check": ([_vp, C.c_int], C.c_int),
     "nfx_divide_check": ([C.c_int, _i64, _vp, _vp, _vp], C.c_int),
     "nfx_indenter_force_noalloc": ([C.c_int, _i64, _vp, C.c_int, C.c_double, C.c_double, C.c_double, _vp, _vp],

@@ -270,6 +270,13 @@ class CellSim:
         check(self._L.nfx_profile_tet_pass(self._h, int(launches), C.byref(ms)))
         return ms.value
 
+    def step_counts(self) -> dict:
+        """Kernel launches of the steps so far, and how many steps went in runs of one launch (up to four
+        and up to six tiles per SM) and by the two passes."""
+        n = (C.c_int64 * 4)()
+        check(self._L.nfx_step_counts(self._h, n))
+        return dict(zip(("launches", "run4", "run6", "passes"), n))
+
     def mesh_info(self) -> tuple[int, int]:
         a, b = C.c_int64(), C.c_int64()
         check(self._L.nfx_mesh_info(self._h, C.byref(a), C.byref(b)))

@@ -93,6 +93,9 @@ struct nfx_sim {
     // Calls that enqueued steps, counted after their launches, and the count up to which the stream was
     // last found idle by another handle (others_busy).
     std::atomic<unsigned long long> work{0}, idle{0};
+    // what the handle's steps were made of so far (nfx_step_counts): launches, steps in runs of either form,
+    // steps in the two passes
+    int64_t n_launches = 0, n_run[2] = {0, 0}, n_passes = 0;
     // Page-locked host memory that kernels write small results into: the readout (first word) and,
     // of small meshes, the positions. The result is there when the stream has been waited for, without
     // a copy behind the kernel.
@@ -221,8 +224,14 @@ int enqueue_steps(nfx_sim* s, int n) {
         CUDA_TRY(launch_nodes(s, k, NODE_UPDATE, -1, true));
     }
     CUDA_TRY(launch_advance_time(s->st, n, s->fields_every, s->record_every, s->stream));
-    s->work++;
     return NFX_OK;
+}
+
+// Notes the n steps of an enqueue_steps, or of a graph of it, as enqueued.
+void note_passes(nfx_sim* s, int64_t n) {
+    s->work++;
+    s->n_passes += n;
+    s->n_launches += n * (s->cell.si_contact >= 0 ? 3 : 2) + 1;
 }
 
 // The barrier's counter back to zero (a run that timed out leaves it anywhere).
@@ -325,12 +334,14 @@ int run_steps(nfx_sim* s, int64_t n) {
         const long long plain = plain_steps(s, t, most);
         if (plain >= RUN_STEPS_MIN) {
             CUDA_TRY(cudaMemsetAsync(s->d_run_acc, 0, 9 * (size_t)s->plan.np * sizeof(unsigned long long), s->stream));
-            CUDA_TRY(launch_run(s->mesh, s->st, table_view(s), s->cell.mat.model,
-                                s->mesh.ntiles <= s->run_tiles[0] ? 0 : 1, s->d_arrivals, s->arrivals, s->d_run_acc,
-                                (int)plain, s->stream));
+            const int form = s->mesh.ntiles <= s->run_tiles[0] ? 0 : 1;
+            CUDA_TRY(launch_run(s->mesh, s->st, table_view(s), s->cell.mat.model, form, s->d_arrivals, s->arrivals,
+                                s->d_run_acc, (int)plain, s->stream));
             s->arrivals += (unsigned)plain * (unsigned)s->mesh.ntiles;
             CUDA_TRY(launch_advance_time(s->st, plain, s->fields_every, s->record_every, s->stream));
             s->work++;
+            s->n_run[form] += plain;
+            s->n_launches += 2;
             done += plain;
         } else {
             // up to the next stretch worth a run: the due steps and the few between them
@@ -339,6 +350,7 @@ int run_steps(nfx_sim* s, int64_t n) {
             k = std::min(k, most);
             const int rc = enqueue_steps(s, (int)k);
             if (rc != NFX_OK) return rc;
+            note_passes(s, k);
             done += k;
         }
     }
@@ -936,10 +948,13 @@ int nfx_step(nfx_sim* s, int64_t nsteps) {
     while (left >= GRAPH_STEPS) {
         if (!s->graph_valid && (rc = build_graph(s)) != NFX_OK) return rc;
         CUDA_TRY(cudaGraphLaunch(s->graph, s->stream));
-        s->work++;
+        note_passes(s, GRAPH_STEPS);
         left -= GRAPH_STEPS;
     }
-    if (left > 0 && (rc = enqueue_steps(s, (int)left)) != NFX_OK) return rc;
+    if (left > 0) {
+        if ((rc = enqueue_steps(s, (int)left)) != NFX_OK) return rc;
+        note_passes(s, left);
+    }
     s->time += nsteps;
     if (nsteps > 0) note_rows(s, t_begin, s->time - 1);
     return NFX_OK;
@@ -1415,6 +1430,15 @@ int nfx_set_plastic_tensor(nfx_sim* s, const double* in) {
     CUDA_TRY(cudaMemcpyAsync(s->d_stage, in, 9 * (size_t)nt * sizeof(double), cudaMemcpyHostToDevice, s->stream));
     CUDA_TRY(launch_plastic_from_user(s->plan.nslots, nt, s->st, s->d_tet_user, s->d_stage, s->stream));
     CUDA_TRY(cudaStreamSynchronize(s->stream));
+    return NFX_OK;
+}
+
+int nfx_step_counts(nfx_sim* s, int64_t* counts) {
+    CHECK_ARG(s && counts, "null argument");
+    counts[0] = s->n_launches;
+    counts[1] = s->n_run[0];
+    counts[2] = s->n_run[1];
+    counts[3] = s->n_passes;
     return NFX_OK;
 }
 

@@ -155,3 +155,23 @@ def test_short_record_intervals_keep_the_graph(fake, material, tiles, every, run
         assert fake.fake_count(RUNS) == 0 and fake.fake_count(GRAPHS) == 4 and fake.fake_count(TETS) == 30
         assert fake.fake_count(ADVANCES) == 1
     s.close()
+
+
+@pytest.mark.parametrize("run_tiles,indenter,every", [((608, 912), "plane", 50), ((4, 912), "plane", 7), ((0, 0), "plane", 50),
+                                                      ((608, 912), "sphere_integral", 50), ((608, 912), "plane", 3)])
+def test_step_counts_are_what_was_launched(fake, run_tiles, indenter, every):
+    fake.fake_run_tiles(*run_tiles)
+    s = cell(indenter=indenter, record_every=every)
+    fake.fake_reset()
+    before = s.step_counts()
+    for n in (1, 3, 57, 430, 0, 12):
+        s.step(n)
+    got = {k: v - before[k] for k, v in s.step_counts().items()}
+    graphs = fake.fake_count(GRAPHS)
+    each = 3 if indenter == "sphere_integral" else 2
+    assert got["passes"] == fake.fake_count(TETS) + 100 * graphs
+    assert got["run4"] + got["run6"] == fake.fake_count(RUN_STEPS) == 503 - got["passes"]
+    assert (got["run4"] > 0) == (run_tiles[0] > 4 and indenter == "plane" and every == 50)
+    assert (got["run6"] > 0) == (run_tiles[0] == 4)
+    assert got["launches"] == sum(fake.fake_count(k) for k in (TETS, NODES, SIS, RUNS, ADVANCES)) + graphs * (100 * each + 1)
+    s.close()
