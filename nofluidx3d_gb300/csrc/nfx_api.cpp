@@ -316,13 +316,14 @@ int use_runs(nfx_sim* s, int64_t nsteps, bool& yes) {
     return NFX_OK;
 }
 
-// Steps from time t on before one that records a row or writes fields (0: that is step t itself).
+// Steps from time t on before one that records a row or writes fields (0: that is step t itself); by
+// remainders, since an interval may be as large as its type.
 long long plain_steps(const nfx_sim* s, long long t, long long most) {
     long long n = most;
     if (s->cell.record_contact >= 0 && s->record_every > 0)
-        n = std::min(n, (t + s->record_every - 1) / s->record_every * s->record_every - t);
+        n = std::min(n, t % s->record_every == 0 ? 0 : s->record_every - t % s->record_every);
     if (s->cell.mat.model == MODEL_VP && s->fields_every > 0)
-        n = std::min(n, (t + s->fields_every) / s->fields_every * s->fields_every - 1 - t);
+        n = std::min(n, s->fields_every - 1 - t % s->fields_every);
     return n;
 }
 

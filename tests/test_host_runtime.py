@@ -175,3 +175,19 @@ def test_step_counts_are_what_was_launched(fake, run_tiles, indenter, every):
     assert (got["run6"] > 0) == (run_tiles[0] == 4)
     assert got["launches"] == sum(fake.fake_count(k) for k in (TETS, NODES, SIS, RUNS, ADVANCES)) + graphs * (100 * each + 1)
     s.close()
+
+
+@pytest.mark.parametrize("material", ["nh", "mr_vp"])
+@pytest.mark.parametrize("every", [2 ** 63 - 1, 2 ** 63 - 2, 2 ** 62])
+def test_record_interval_at_the_end_of_its_range(fake, material, every):
+    """An interval that never comes, up to the largest: each step is enqueued once, the due ones by the passes."""
+    fake.fake_run_tiles(608, 912)
+    s = cell(material=material)
+    s.set_record(1, every, 10)
+    fake.fake_reset()
+    for n in (10, 100, 7):  # step 0 records a row
+        s.step(n)
+        assert fake.fake_count(ADVANCES) < 20
+    assert s.time == 117
+    assert fake.fake_count(RUN_STEPS) == 116 and fake.fake_count(TETS) == 1
+    s.close()
