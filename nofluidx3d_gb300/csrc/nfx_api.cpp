@@ -49,6 +49,19 @@ constexpr size_t HOST_OUT = 4096;
 
 void nfx::set_error(const std::string& msg) { g_err = msg; }
 
+nfx::Workers& nfx::workers() {
+    static Workers* w = new Workers;  // never freed: handles may be destroyed while the process exits
+    return *w;
+}
+void nfx::Workers::add(Worker* w) {
+    std::lock_guard<std::mutex> hold(lock);
+    all.push_back(w);
+}
+void nfx::Workers::remove(Worker* w) {
+    std::lock_guard<std::mutex> hold(lock);
+    all.erase(std::remove(all.begin(), all.end(), w), all.end());
+}
+
 struct nfx_sim {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -90,9 +103,7 @@ struct nfx_sim {
     unsigned arrivals = 0;
     int run_tiles[2] = {-1, -1};
     unsigned long long* d_run_acc = nullptr;  // three accumulators, allocated with a mesh that may take runs
-    // Calls that enqueued steps, counted after their launches, and the count up to which the stream was
-    // last found idle by another handle (others_busy).
-    std::atomic<unsigned long long> work{0}, idle{0};
+    Worker worker;
     // what the handle's steps were made of so far (nfx_step_counts): launches, steps in runs of either form,
     // steps in the two passes
     int64_t n_launches = 0, n_run[2] = {0, 0}, n_passes = 0;
@@ -229,7 +240,7 @@ int enqueue_steps(nfx_sim* s, int n) {
 
 // Notes the n steps of an enqueue_steps, or of a graph of it, as enqueued.
 void note_passes(nfx_sim* s, int64_t n) {
-    s->work++;
+    s->worker.work++;
     s->n_passes += n;
     s->n_launches += n * (s->cell.si_contact >= 0 ? 3 : 2) + 1;
 }
@@ -245,18 +256,6 @@ int reset_arrivals(nfx_sim* s) {
 // accumulators and the loading of the tiles (about 6 us, a step of the two passes) once.
 constexpr int RUN_STEPS_MIN = 4, RUN_STEPS_MAX = 1024;
 
-// The process's handles (never freed: handles may be destroyed while the process exits). The lock is held
-// while a stream is captured, so that no other handle queries it then, and until a handle is out of
-// the list before its stream goes.
-struct Handles {
-    std::mutex lock;
-    std::vector<nfx_sim*> all;
-};
-Handles& handles() {
-    static Handles* h = new Handles;
-    return *h;
-}
-
 // Calls that another thread's capture in the strict mode would forbid to every thread, but do it no harm.
 struct RelaxedCapture {
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
@@ -269,10 +268,10 @@ struct RelaxedCapture {
 // at most 32 are asked.
 bool others_busy(const nfx_sim* s) {
     RelaxedCapture relaxed;
-    std::lock_guard<std::mutex> hold(handles().lock);
+    std::lock_guard<std::mutex> hold(workers().lock);
     int asked = 0;
-    for (nfx_sim* o : handles().all) {
-        if (o == s || o->device != s->device) continue;
+    for (Worker* o : workers().all) {
+        if (o == &s->worker || o->device != s->device) continue;
         const unsigned long long work = o->work.load();
         if (work == o->idle.load()) continue;
         if (cudaStreamQuery(o->stream) == cudaErrorNotReady) {
@@ -311,7 +310,10 @@ int use_runs(nfx_sim* s, int64_t nsteps, bool& yes) {
     if (s->run_tiles[0] < 0) CUDA_TRY(run_tiles_max(s->mesh, s->cell.mat.model, s->run_tiles));
     yes = s->mesh.ntiles <= std::max(s->run_tiles[0], s->run_tiles[1]) && longest_stretch(s) >= stretch_min(s);
     // Runs of cells of which fewer than four fit the GPU side by side take turns, while the two passes of
-    // several handles overlap: four R = 14 cells stepped by four threads 53 ms in runs, 32 in passes.
+    // several handles overlap: four R = 14 cells stepped by four threads 53 ms in runs, 32 in passes. And
+    // they leave a batch beside them no SMs while they last: 4000 steps of an R = 14 cell and 2000 of 64
+    // small cells in two threads, each done after 33 and 55 ms in runs, 56 and 34 in passes (59 and 36
+    // before there were runs).
     if (yes && 4 * s->mesh.ntiles > s->run_tiles[0] && others_busy(s)) yes = false;
     return NFX_OK;
 }
@@ -340,7 +342,7 @@ int run_steps(nfx_sim* s, int64_t n) {
                                 s->d_run_acc, (int)plain, s->stream));
             s->arrivals += (unsigned)plain * (unsigned)s->mesh.ntiles;
             CUDA_TRY(launch_advance_time(s->st, plain, s->fields_every, s->record_every, s->stream));
-            s->work++;
+            s->worker.work++;
             s->n_run[form] += plain;
             s->n_launches += 2;
             done += plain;
@@ -361,7 +363,7 @@ int run_steps(nfx_sim* s, int64_t n) {
 int build_graph(nfx_sim* s) {
     invalidate_graph(s);
     cudaGraph_t g = nullptr;
-    std::lock_guard<std::mutex> hold(handles().lock);
+    std::lock_guard<std::mutex> hold(workers().lock);
     CUDA_TRY(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
     int rc = enqueue_steps(s, GRAPH_STEPS);
     cudaError_t e = cudaStreamEndCapture(s->stream, &g);
@@ -568,21 +570,16 @@ int nfx_create(int device, nfx_sim** out) {
     s->cell.vv_a = (float)((1 - 0.5 * xi) / (1 + 0.5 * xi));
     s->cell.vv_hb = (float)(0.5 / (1 + 0.5 * xi));
     s->cell.vv_dm = (float)(1 - 0.5 * xi);
-    {
-        std::lock_guard<std::mutex> hold(handles().lock);
-        handles().all.push_back(s);
-    }
+    s->worker.device = device;
+    s->worker.stream = s->stream;
+    workers().add(&s->worker);
     *out = s;
     return NFX_OK;
 }
 
 int nfx_destroy(nfx_sim* s) {
     if (!s) return NFX_OK;
-    {
-        std::lock_guard<std::mutex> hold(handles().lock);
-        std::vector<nfx_sim*>& all = handles().all;
-        all.erase(std::remove(all.begin(), all.end(), s), all.end());
-    }
+    workers().remove(&s->worker);
     cudaSetDevice(s->device);
     if (s->stream) cudaStreamSynchronize(s->stream);
     invalidate_graph(s);
@@ -1309,7 +1306,7 @@ int nfx_run_timeout_check(nfx_sim* s, int polls) {
                         s->d_arrivals, s->arrivals + 1, s->d_run_acc, RUN_STEPS_MIN, s->stream, (unsigned)polls));
     s->arrivals += (unsigned)RUN_STEPS_MIN * (unsigned)s->mesh.ntiles;
     CUDA_TRY(launch_advance_time(s->st, RUN_STEPS_MIN, s->fields_every, s->record_every, s->stream));
-    s->work++;
+    s->worker.work++;
     s->time += RUN_STEPS_MIN;
     return NFX_OK;
 }

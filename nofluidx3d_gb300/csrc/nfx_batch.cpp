@@ -121,6 +121,7 @@ struct nfx_batch {
     std::vector<int> tuned_bucket;
     long long* d_zero_meta = nullptr;
     bool has_si = false;  // some cell has an integrated sphere contact
+    Worker worker;
 };
 
 namespace {
@@ -472,6 +473,7 @@ int batch_step(nfx_batch* b, BatchDevice& D, int64_t nsteps) {
     while (left >= BATCH_GRAPH_STEPS) {
         if (!D.graph) {
             cudaGraph_t g = nullptr;
+            std::lock_guard<std::mutex> hold(workers().lock);
             BCUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
             int rc = enqueue_batch_steps(b, D, BATCH_GRAPH_STEPS);
             cudaError_t e = cudaStreamEndCapture(b->stream, &g);
@@ -485,9 +487,14 @@ int batch_step(nfx_batch* b, BatchDevice& D, int64_t nsteps) {
             if (e != cudaSuccess) return bfail(NFX_ERR_CUDA, std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e));
         }
         BCUDA(cudaGraphLaunch(D.graph, b->stream));
+        b->worker.work++;
         left -= BATCH_GRAPH_STEPS;
     }
-    if (left > 0) return enqueue_batch_steps(b, D, (int)left);
+    if (left > 0) {
+        const int rc = enqueue_batch_steps(b, D, (int)left);
+        if (rc != NFX_OK) return rc;
+        b->worker.work++;
+    }
     return NFX_OK;
 }
 
@@ -598,12 +605,16 @@ int nfx_batch_create(int device, int tile_tets, nfx_batch** out) {
     }
     cudaMemset(z, 0, 2 * sizeof(long long));
     b->d_zero_meta = (long long*)z;
+    b->worker.device = device;
+    b->worker.stream = b->stream;
+    workers().add(&b->worker);
     *out = b;
     return NFX_OK;
 }
 
 int nfx_batch_destroy(nfx_batch* b) {
     if (!b) return NFX_OK;
+    workers().remove(&b->worker);
     cudaSetDevice(b->device);
     if (b->stream) cudaStreamSynchronize(b->stream);
     b->dev.release();

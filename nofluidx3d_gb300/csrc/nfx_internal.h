@@ -1,7 +1,9 @@
 // Internal data structures shared by the host runtime (nfx_api.cpp, nfx_mesh.cpp) and the
 // kernels (nfx_kernels.cu). Not part of the C ABI.
 #pragma once
+#include <atomic>
 #include <functional>
+#include <mutex>
 #include <cuda_runtime.h>
 #include <nvtx3/nvToolsExt.h>
 
@@ -83,6 +85,23 @@ struct MeshPlan {
     bool all_nodes_used = false;           // every node belongs to a tetra
     float fix_max = FORCE_FIX_MAX;         // per-tile fixed-point bound, force_fix_bound(max_tiles_per_node)
 };
+
+// A handle's stream as other handles see it: calls that enqueued steps, counted after their launches, and
+// the count up to which the stream was last found idle by another handle.
+struct Worker {
+    int device = 0;
+    cudaStream_t stream = nullptr;
+    std::atomic<unsigned long long> work{0}, idle{0};
+};
+// The process's workers, cells' and batches'. The lock is held while a stream is captured, so that no
+// other handle queries it then, and until a worker is out of the list before its stream goes.
+struct Workers {
+    std::mutex lock;
+    std::vector<Worker*> all;
+    void add(Worker* w);
+    void remove(Worker* w);
+};
+Workers& workers();
 
 // Runs work(b0, b1) over [0, n) on up to `threads` host threads, at least 4 items each. False when a
 // part ran out of memory (an exception must not leave its thread).

@@ -4,7 +4,7 @@ it, and by the two passes elsewhere — so that a comparison of the two is one."
 import numpy as np
 import pytest
 
-from nofluidx3d_gb300.core import CellSim
+from nofluidx3d_gb300.core import Batch, CellSim
 from nofluidx3d_gb300.workloads import Workload
 
 pytestmark = pytest.mark.gpu
@@ -59,3 +59,22 @@ def test_loaded_device_changes_the_way_of_larger_cells_only():
     assert s.step_counts()["run4"] >= 40
     for t in (busy, s, small):
         t.close()
+
+
+def test_larger_cells_give_way_to_a_batch():
+    w = Workload("ways", radius=13.0, material="nh", indenter="sphere", sphere_radius=4.0, speed=2e-3)
+    batch, s = Batch(0, 128), CellSim(0)
+    for r in (4.0, 5.0, 6.0):
+        w.with_(radius=r).add_to_batch(batch)
+    batch.set_record(1, 50, 1000)
+    batch.finalize()
+    w.configure(s, max_rows=500)
+    s.sync()
+    batch.step(20000)  # some 0.1 s of work
+    s.step(50)
+    assert s.step_counts()["passes"] == 50
+    batch.status()  # waits for the batch
+    s.step(50)
+    assert s.step_counts()["run4"] >= 40
+    batch.close()
+    s.close()
